@@ -202,7 +202,8 @@ typedef struct {
     int32_t storage;        /* JT_STORE_* of the node values                  */
     int32_t n_pairs;
     int32_t near_degenerate; /* nonzero: tet_box flags some tetrahedra (jt_mark_near_degenerate) */
-    int32_t pad;
+    int32_t locator;        /* 0, or what jt_mesh_locator_build returned: a
+                               locator block follows dtab                     */
     int64_t pair_stride;    /* records per pair (= n_points)                  */
     const float* points;    /* device (n_points,4): x,y,z,0                   */
     const float* tet_box;   /* device (n_tets,8): min xyz,flag, max xyz,0 (flag: jt_mark_near_degenerate) */
@@ -217,10 +218,28 @@ typedef struct {
      * octants (0 for a leaf) and first the breadth-first index of the first
      * child (< 2^24); dtab (n_nodes,2) holds the node's elem_offset and
      * elem_count.  One 16-byte load per level instead of two dependent
-     * loads, the same moves as the node records. */
+     * loads, the same moves as the node records.  With `locator` set, dtab
+     * points to jt_mesh_locator_bytes bytes that jt_mesh_locator_build
+     * filled behind the n_nodes rows (64-byte aligned). */
     const int32_t* desc;
     const int32_t* dtab;
 } jt_mesh_field;
+
+/* Locator of a mesh field (no counterpart in the reference: it replaces the
+ * top of the descent and the gather of the leaf's tetrahedra, with the same
+ * candidates in the same order).  Every node of one level splits an axis at
+ * the same float32 centre when it has the same path on that axis, so the
+ * first `depth` moves of a descent are three bracketing searches among 2^depth
+ * cells and one table entry; jt_mesh_locator_build compares each centre on
+ * the way with `splits` and refuses a tree for which this does not hold.
+ *   jt_mesh_locator_bytes: size of the buffer dtab has to point to.
+ *   jt_mesh_locator_build: fills it behind dtab's rows.  m: desc, dtab, elems
+ *     and tet_geom set; n_entries: length of elems; depth 1..7, at most
+ *     max_depth; splits: device (3, 2^depth + 1) float32, ascending, the cell
+ *     faces of each axis (the outer two are not compared).  *locator_out (host)
+ *     receives the value for jt_mesh_field.locator, 0 where the tree does not
+ *     split so (the buffer is then not used).  Synchronises the stream. */
+#define JT_MESH_LOCATOR_MAX_DEPTH 7
 
 /* Nearest-node field: TimeSeriesField spatial sampling (time_series.py:391)
  * over scattered nodes, accelerated by a uniform cell list. */
@@ -650,6 +669,11 @@ int jt_octree_build_device(const float* points, int32_t n_points, const int32_t*
  * NULL) receives the number flagged.  Returns after the pass has finished. */
 int jt_mark_near_degenerate(float* tet_box, const float* tet_geom, int32_t n_tets, int32_t* count_out,
                             void* stream);
+
+/* Locator block of a mesh field (see jt_mesh_field): size, and build. */
+size_t jt_mesh_locator_bytes(int32_t n_nodes, int32_t n_entries, int32_t depth);
+int jt_mesh_locator_build(const jt_mesh_field* m, int32_t n_entries, int32_t depth, const float* splits,
+                          int32_t* locator_out, void* stream);
 
 /* Copy the device build's nodes (n_nodes) and node_bounds (n_nodes,6) into
  * caller buffers (device or host; either may be NULL), ordered on `stream`. */

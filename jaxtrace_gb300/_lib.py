@@ -29,6 +29,7 @@ JT_EULER, JT_RK2, JT_RK4 = 0, 1, 2
 JT_BC_NONE, JT_BC_PERIODIC, JT_BC_REFLECTIVE, JT_BC_CLAMP, JT_BC_ABSORBING = 0, 1, 2, 3, 4
 JT_INLET_OFF, JT_INLET_GRID = 0, 1
 JT_ARITH_EXACT, JT_ARITH_COMPENSATED = 0, 1
+JT_MESH_LOCATOR_MAX_DEPTH = 7
 JT_FIELD_GRID, JT_FIELD_MESH, JT_FIELD_NEAREST, JT_FIELD_FEM = 1, 2, 3, 4
 
 STORAGE_CODES = {"f32": JT_STORE_F32, "float32": JT_STORE_F32, "bf16": JT_STORE_BF16,
@@ -63,7 +64,7 @@ OCTREE_NODE_DTYPE = np.dtype([("c", "<f4", (3,)), ("is_leaf", "<i4"), ("children
 
 class MeshField(C.Structure):
     _fields_ = [("n_points", i32), ("n_tets", i32), ("n_nodes", i32), ("max_depth", i32),
-                ("storage", i32), ("n_pairs", i32), ("near_degenerate", i32), ("pad", i32), ("pair_stride", i64),
+                ("storage", i32), ("n_pairs", i32), ("near_degenerate", i32), ("locator", i32), ("pair_stride", i64),
                 ("points", vp), ("tet_box", vp), ("tet_geom", vp), ("nodes", vp), ("elems", vp),
                 ("pairs", vp), ("desc", vp), ("dtab", vp)]
 
@@ -181,6 +182,8 @@ def load(build_if_missing: bool = True):
         "jt_octree_fetch_device": (i32, [vp, vp, vp, vp]),
         "jt_octree_free_device": (None, [vp, vp]),
         "jt_mark_near_degenerate": (i32, [vp, vp, i32, P(i32), vp]),
+        "jt_mesh_locator_bytes": (C.c_size_t, [i32, i32, i32]),
+        "jt_mesh_locator_build": (i32, [P(MeshField), i32, i32, vp, P(i32), vp]),
         "jt_pair_log_ratio": (i32, [vp, vp, i32, f32, vp, vp, vp]),
         "jt_fem_grid_build": (i32, [vp, i32, vp, i32, vp, vp, vp, i32, vp, P(vp), P(FemGridInfo)]),
         "jt_fem_grid_fetch": (i32, [vp, vp, vp, vp, vp]),

@@ -8,6 +8,7 @@
 #include "jt_common.cuh"
 #include "jt_internal.h"
 #include "jt_kernels.cuh"
+#include "jt_mesh.cuh"
 
 namespace jt {
 
@@ -112,6 +113,9 @@ static int check_field(const jt_field* f) {
                 m->elems == nullptr || m->pairs == nullptr || m->n_pairs < 1)
                 return set_error(JT_ERR_INVALID, "mesh field has a NULL array");
             if (m->max_depth < 0) return set_error(JT_ERR_INVALID, "max_depth must be >= 0");
+            // a locator's depth lies in the word's low byte; any other value there is ignored
+            if (locator_depth(*m) > 0 && (m->desc == nullptr || m->dtab == nullptr || ((uintptr_t)m->dtab & 63u) != 0))
+                return set_error(JT_ERR_INVALID, "a mesh locator needs desc and a 64-byte aligned dtab");
             if (m->pair_stride < m->n_points) return set_error(JT_ERR_INVALID, "pair_stride smaller than n_points");
             if (((uintptr_t)m->pairs & 31u) != 0)
                 return set_error(JT_ERR_INVALID, "pairs must be 32-byte aligned (256-bit records)");

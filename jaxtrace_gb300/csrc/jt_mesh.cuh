@@ -99,6 +99,102 @@ __device__ __forceinline__ bool tet_bary(const V3& q, const float* tet_box, cons
     return true;
 }
 
+// ---------------------------------------------------------------------------
+// Locator block (jt_mesh_locator_build), behind the dtab rows:
+//   header  8 floats: origin xyz, cells per unit xyz, 0, mismatch flag (build)
+//   faces   per axis 2^D {lower, upper} faces of its cells, the outer ones
+//           NaN (nothing is below or above them)
+//   table   8^D {elem_offset, elem_count} of the node that D moves reach, or
+//           {breadth-first node, -1} where the descent goes on below it
+//   slots   64 B per element-list slot: the tetrahedron's tet_geom record,
+//           its first vertex id with the top bit set where the tetrahedron is
+//           well shaped (kWellShaped)
+// All offsets are multiples of 64 B from the 64-aligned end of dtab's rows.
+//
+// Why: the evaluation was held by the L1 (93 % busy) on 34 gathers per query,
+// seven of them the levels of the descent and six per candidate (list entry,
+// two halves of the box, three quarters of the geometry).  The table takes the
+// descent to four independent loads and one dependent one, and the slot order
+// the candidate to two 256-bit loads of one line.  1M particles x 64 steps on
+// 1,572,864 tetrahedra (64^3 hexahedra): tracking kernel 15.6 -> 12.8 ms;
+// 24 ensembles x 50 steps 7.1 -> 5.6 ms; same bits.
+// ---------------------------------------------------------------------------
+constexpr int32_t kLocatorMagic = 0x4a544c00;  // jt_mesh_field.locator = magic | depth
+
+struct LocatorLayout {
+    size_t header, faces, table, slots, bytes;
+};
+
+__host__ __device__ inline LocatorLayout locator_layout(int64_t n_nodes, int64_t n_entries, int depth) {
+    auto al = [](size_t b) { return (b + 63) & ~(size_t)63; };
+    LocatorLayout o;
+    o.header = al((size_t)n_nodes * 8);
+    o.faces = o.header + 64;
+    o.table = al(o.faces + ((size_t)3 << depth) * 8);
+    o.slots = al(o.table + ((size_t)8 << (3 * depth)));
+    o.bytes = o.slots + (size_t)n_entries * 64;
+    return o;
+}
+
+__host__ __device__ inline int locator_depth(const jt_mesh_field& F) {
+    const int d = F.locator & 0xff;
+    return (F.locator & ~0xff) == kLocatorMagic && d >= 1 && d <= JT_MESH_LOCATOR_MAX_DEPTH ? d : 0;
+}
+
+// A tetrahedron is well shaped when the cube of its longest edge is at most
+// kWellShaped |det|.  The float32 barycentrics of a query near it are then off
+// by less than 64 * 2^-24 * kWellShaped = 4.9e-4: each numerator is six triple
+// products of components no longer than that edge, three roundings each and
+// five in the sum.  kInside is twice that, so a query whose computed
+// barycentrics are all at least kInside lies inside the tetrahedron, at least
+// 4.9e-4 of the box's extent away from each of its faces, and the box test,
+// whose faces are the vertices' own floats, cannot fail: it is left out.
+constexpr float kWellShaped = 128.0f;
+constexpr float kInside = 1e-3f;
+
+__device__ __forceinline__ bool well_shaped(const float* g12) {
+    const V3 a{g12[3], g12[4], g12[5]}, b{g12[6], g12[7], g12[8]}, c{g12[9], g12[10], g12[11]};
+    const float det = fabsf(det3<true>(a, b, c));
+    const float la = a.x * a.x + a.y * a.y + a.z * a.z, lb = b.x * b.x + b.y * b.y + b.z * b.z;
+    const float lc = c.x * c.x + c.y * c.y + c.z * c.z;
+    const float l = sqrtf(fmaxf(fmaxf(la, lb), lc));
+    return det >= 1e-10f && l * l * l <= kWellShaped * det;
+}
+
+// The barycentric test of one 64-byte record (tet_bary without the box test).
+// A candidate that is clearly outside is rejected on the numerators, before
+// the three divisions: b = numerator / det is below -1.9e-6 or above 1.00001
+// there, well past the -1e-6 and 0.999999 it is compared with, so the answer
+// is that of the divided values.  Comparisons with NaN reject nothing and
+// leave the decision to the full test.
+template <bool EXACT>
+__device__ __forceinline__ bool slot_bary(const V3& q, const uint32_t (&g0)[8], const uint32_t (&g1)[8], float4& b) {
+    typedef Ar<EXACT> A;
+    const auto f = [](uint32_t w) { return __uint_as_float(w); };
+    const V3 v01{f(g0[3]), f(g0[4]), f(g0[5])}, v02{f(g0[6]), f(g0[7]), f(g1[0])}, v03{f(g1[1]), f(g1[2]), f(g1[3])};
+    const V3 p{A::sub(q.x, f(g0[0])), A::sub(q.y, f(g0[1])), A::sub(q.z, f(g0[2]))};
+    float det = det3<EXACT>(v01, v02, v03);
+    if (fabsf(det) < 1e-10f) det = 1.0f;
+    const float ad = fabsf(det), lo = -2e-6f * ad, hi = 1.00001f * ad;
+    const uint32_t sg = __float_as_uint(det) & 0x80000000u;
+    const auto signed_by = [sg](float v) { return __uint_as_float(__float_as_uint(v) ^ sg); };
+    const float ny = det3<EXACT>(p, v02, v03);
+    const float sy = signed_by(ny);
+    if (sy < lo || sy > hi) return false;
+    const float nz = det3<EXACT>(v01, p, v03);
+    const float sz = signed_by(nz);
+    if (sz < lo || sy + sz > hi) return false;
+    const float nw = det3<EXACT>(v01, v02, p);
+    const float sw = signed_by(nw);
+    if (sw < lo || sy + sz + sw > hi) return false;
+    b.y = A::div(ny, det);
+    b.z = A::div(nz, det);
+    b.w = A::div(nw, det);
+    b.x = A::sub(A::sub(A::sub(1.0f, b.y), b.z), b.w);
+    const float l = -1e-6f, h = 0.999999f;  // tol and 1 + tol as float32
+    return b.x >= l && b.y >= l && b.z >= l && b.w >= l && b.x <= h && b.y <= h && b.z <= h && b.w <= h;
+}
+
 // jnp.dot(bary, node_values): terms accumulated in vertex order.
 template <bool EXACT>
 __device__ __forceinline__ V3 p1_combine(const float4& b, const V3& n0, const V3& n1, const V3& n2, const V3& n3) {
@@ -121,8 +217,87 @@ struct MeshFieldT {
     // registers, no spills) keep more warps in flight than the default 3
     static constexpr int kMinBlocks = JT_MESH_MIN_BLOCKS;
     jt_mesh_field F;
+    const char* loc;      // locator block's header, or NULL
+    int depth;            // its depth
+    uint32_t faces, table, slots;  // offsets from the header
 
-    static MeshFieldT create(const jt_mesh_field& d, int) { return MeshFieldT{d}; }
+    static MeshFieldT create(const jt_mesh_field& d, int) {
+        MeshFieldT m{d, nullptr, locator_depth(d), 0, 0, 0};
+        if (m.depth > 0) {
+            const LocatorLayout o = locator_layout(d.n_nodes, 0, m.depth);
+            m.loc = reinterpret_cast<const char*>(d.dtab) + o.header;
+            m.faces = (uint32_t)(o.faces - o.header);
+            m.table = (uint32_t)(o.table - o.header);
+            m.slots = (uint32_t)(o.slots - o.header);
+        }
+        return m;
+    }
+
+    // Cell of coordinate x among the 2^depth cells of axis a: the number of
+    // split centres at or below x, which is what the descent's comparisons
+    // x >= centre add up to.  The guess is off by one only within rounding
+    // of a face; NaN stays in cell 0, as every comparison of the descent fails.
+    __device__ __forceinline__ int face_cell(float x, float org, float inv, int a) const {
+        const int n = 1 << depth;
+        int g = (int)fminf(fmaxf((x - org) * inv, 0.0f), (float)(n - 1));
+        const float2* f = reinterpret_cast<const float2*>(loc + faces) + (a << depth);
+        float2 b = __ldg(f + g);
+        while (x < b.x) b = __ldg(f + --g);   // ends at the NaN of cell 0
+        while (x >= b.y) b = __ldg(f + ++g);  // ends at the NaN of the last cell
+        return g;
+    }
+
+    // The leaf (or dead end) of the descent, {elem_offset, elem_count}.
+    __device__ __forceinline__ int2 locate(const V3& q) const {
+        const float4 h0 = __ldg(reinterpret_cast<const float4*>(loc));
+        const float2 h1 = __ldg(reinterpret_cast<const float2*>(loc) + 2);
+        const int ix = face_cell(q.x, h0.x, h0.w, 0), iy = face_cell(q.y, h0.y, h1.x, 1);
+        const int iz = face_cell(q.z, h0.z, h1.y, 2);
+        const int2 oc = __ldg(reinterpret_cast<const int2*>(loc + table) + ((((ix << depth) | iy) << depth) | iz));
+        return oc.y >= 0 ? oc : descend(q, oc.x, depth);
+    }
+
+    // Descent on the breadth-first copy from `node`, which `d` moves reached:
+    // a child's index is the node's first child plus the present octants below
+    // its own.
+    __device__ __forceinline__ int2 descend(const V3& q, int node, int d) const {
+        const int4* D = reinterpret_cast<const int4*>(F.desc);
+        for (; d < F.max_depth; ++d) {
+            const int4 h = __ldg(D + node);
+            const unsigned w = (unsigned)h.w, m = w & 0xffu;
+            if (m == 0u) break;  // a leaf (or a node without children)
+            const int oct = (q.x >= __int_as_float(h.x) ? 1 : 0) + (q.y >= __int_as_float(h.y) ? 2 : 0) +
+                            (q.z >= __int_as_float(h.z) ? 4 : 0);
+            if (!((m >> oct) & 1u)) break;
+            node = (int)(w >> 8) + __popc(m & ((1u << oct) - 1u));
+        }
+        return __ldg(reinterpret_cast<const int2*>(F.dtab) + node);
+    }
+
+    // First candidate of the list that holds the query (…optimized.py:309-360),
+    // its P1 value in v; false when there is none.
+    __device__ __forceinline__ bool scan_slots(const V3& q, int2 oc, const jt_blend& e, V3& v) const {
+        const char* rec = loc + slots + (int64_t)oc.x * 64;
+        for (int s = 0; s < oc.y; ++s, rec += 64) {
+            uint32_t g0[8], g1[8];
+            ldg256(rec, g0);
+            ldg256(rec + 32, g1);
+            float4 b;
+            if (!slot_bary<EXACT>(q, g0, g1, b)) continue;
+            const bool inside = (int)g1[4] < 0 && fminf(fminf(b.x, b.y), fminf(b.z, b.w)) >= kInside;
+            if (!inside || (NEAR && !EXACT)) {
+                const int t = __ldg(F.elems + oc.x + s);
+                const float4* bx = reinterpret_cast<const float4*>(F.tet_box) + 2 * (int64_t)t;
+                const float4 mn = __ldg(bx), mx = __ldg(bx + 1);
+                if (!(q.x >= mn.x && q.y >= mn.y && q.z >= mn.z && q.x <= mx.x && q.y <= mx.y && q.z <= mx.z)) continue;
+                if (NEAR && !EXACT && mn.w != 0.0f) b = bary_f64(q, F.tet_geom, t);
+            }
+            v = p1_combine<EXACT>(b, node_value((int)(g1[4] & 0x7fffffffu), e), node_value((int)g1[5], e),
+                                  node_value((int)g1[6], e), node_value((int)g1[7], e));
+            return true;
+        }
+        return false;
+    }
 
     __device__ __forceinline__ V3 node_value(int node, const jt_blend& e) const {
         const int64_t base = (int64_t)min(max(e.pair, 0), F.n_pairs - 1) * F.pair_stride;
@@ -132,54 +307,46 @@ struct MeshFieldT {
     __device__ __forceinline__ V3 operator()(const V3& q, const jt_blend& e, int& flags) const {
         typedef Ar<EXACT> A;
         // fixed-depth descent (…optimized.py:278-302): at most max_depth moves,
-        // stopping at a leaf or where the query's octant has no child
-        int node = 0;
-        int2 oc;
-        if (F.desc != nullptr) {
-            // the same moves on the breadth-first copy: a child's index is the
-            // node's first child plus the present octants below its own
-            const int4* D = reinterpret_cast<const int4*>(F.desc);
-            for (int d = 0; d < F.max_depth; ++d) {
-                const int4 h = __ldg(D + node);
-                const unsigned w = (unsigned)h.w, m = w & 0xffu;
-                if (m == 0u) break;  // a leaf (or a node without children)
-                const int oct = (q.x >= __int_as_float(h.x) ? 1 : 0) + (q.y >= __int_as_float(h.y) ? 2 : 0) +
-                                (q.z >= __int_as_float(h.z) ? 4 : 0);
-                if (!((m >> oct) & 1u)) break;
-                node = (int)(w >> 8) + __popc(m & ((1u << oct) - 1u));
-            }
-            oc = __ldg(reinterpret_cast<const int2*>(F.dtab) + node);
-        } else {
-            for (int d = 0; d < F.max_depth; ++d) {
-                const int4 h = __ldg(reinterpret_cast<const int4*>(F.nodes + node));
-                if (h.w) break;  // is_leaf
-                const int oct = (q.x >= __int_as_float(h.x) ? 1 : 0) + (q.y >= __int_as_float(h.y) ? 2 : 0) +
-                                (q.z >= __int_as_float(h.z) ? 4 : 0);
-                const int ch = __ldg(&F.nodes[node].children[oct]);
-                if (ch < 0) break;
-                node = ch;
-            }
-            oc = __ldg(reinterpret_cast<const int2*>(&F.nodes[node].elem_offset));
-        }
-        const int32_t* L = F.elems + oc.x;
-        const int cnt = oc.y;
-        // candidate scan (…optimized.py:309-360): first candidate whose box
+        // stopping at a leaf or where the query's octant has no child; then
+        // the candidate scan (…optimized.py:309-360): first candidate whose box
         // holds the query and whose barycentrics pass the tolerance test
-        for (int s = 0; s < cnt; ++s) {
-            float4 b;
-            int4 cn;
-            bool near;
-            const int t = __ldg(L + s);
-            if (!tet_bary<EXACT>(q, F.tet_box, F.tet_geom, t, b, cn, near)) continue;
-            if (NEAR && !EXACT && near) b = bary_f64(q, F.tet_geom, t);
-            return p1_combine<EXACT>(b, node_value(cn.x, e), node_value(cn.y, e), node_value(cn.z, e),
-                                     node_value(cn.w, e));
+        int2 oc;
+        if (loc != nullptr) {
+            oc = locate(q);
+            V3 v;
+            if (scan_slots(q, oc, e, v)) return v;
+        } else {
+            if (F.desc != nullptr) {
+                oc = descend(q, 0, 0);
+            } else {
+                int node = 0;
+                for (int d = 0; d < F.max_depth; ++d) {
+                    const int4 h = __ldg(reinterpret_cast<const int4*>(F.nodes + node));
+                    if (h.w) break;  // is_leaf
+                    const int oct = (q.x >= __int_as_float(h.x) ? 1 : 0) + (q.y >= __int_as_float(h.y) ? 2 : 0) +
+                                    (q.z >= __int_as_float(h.z) ? 4 : 0);
+                    const int ch = __ldg(&F.nodes[node].children[oct]);
+                    if (ch < 0) break;
+                    node = ch;
+                }
+                oc = __ldg(reinterpret_cast<const int2*>(&F.nodes[node].elem_offset));
+            }
+            for (int s = 0; s < oc.y; ++s) {
+                float4 b;
+                int4 cn;
+                bool near;
+                const int t = __ldg(F.elems + oc.x + s);
+                if (!tet_bary<EXACT>(q, F.tet_box, F.tet_geom, t, b, cn, near)) continue;
+                if (NEAR && !EXACT && near) b = bary_f64(q, F.tet_geom, t);
+                return p1_combine<EXACT>(b, node_value(cn.x, e), node_value(cn.y, e), node_value(cn.z, e),
+                                         node_value(cn.w, e));
+            }
         }
         // cheap fallback (…optimized.py:364-376): nearest of the four vertices
         // of the first candidate; an empty list reads slot -1, which indexes
         // the last tetrahedron
         flags |= JT_STATUS_OCTREE_FALLBACK;
-        int first = cnt > 0 ? __ldg(L) : -1;
+        int first = oc.y > 0 ? __ldg(F.elems + oc.x) : -1;
         if (first < 0) first += F.n_tets;
         const int4 cn = __ldg(reinterpret_cast<const int4*>(F.tet_geom) + 4 * (int64_t)first + 3);
         const int ids[4] = {cn.x, cn.y, cn.z, cn.w};

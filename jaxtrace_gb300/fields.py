@@ -947,6 +947,20 @@ def breadth_first_descent(nodes: np.ndarray):
     return desc, dtab
 
 
+def locator_splits(lo, hi, depth: int):
+    """(3, 2^depth + 1) float32 faces of the cells that the first ``depth``
+    levels of an octree over [lo, hi] cut each axis into, the float32 centres
+    (min + max) / 2 of the builders; None where they do not ascend (a box so
+    thin that centres coincide still ascends; one that overflows does not)."""
+    S = np.zeros((3, (1 << depth) + 1), dtype=F32)
+    S[:, 0], S[:, -1] = lo, hi
+    with np.errstate(over="ignore", invalid="ignore"):
+        for level in range(depth):
+            step = 1 << (depth - level)
+            S[:, step // 2::step] = (S[:, :-1:step] + S[:, step::step]) / F32(2.0)
+        return S if np.all(np.diff(S, axis=1) >= 0) else None
+
+
 class OctreeMesh:
     """The octree in the reference's array layout (OctreeMeshOptimized,
     octree_fem_interpolator_optimized.py:18-38).
@@ -1107,10 +1121,31 @@ class OctreeFEMTimeSeriesFieldOptimized(_DeviceField):
         f.near_degenerate = int(self.n_near_degenerate > 0)
         bfs = breadth_first_descent(m.nodes)
         if bfs is not None:
-            d["desc"], d["dtab"] = (torch.from_numpy(a).cuda() for a in bfs)
-            f.desc, f.dtab = d["desc"].data_ptr(), d["dtab"].data_ptr()
+            self._upload_descent(f, d, bfs)
         self._cmesh = f
         self._cfield = L.Field(kind=L.JT_FIELD_MESH, mesh=C.pointer(f))
+
+    def _upload_descent(self, f, d, bfs):
+        """The breadth-first tree, and behind it the locator block
+        (jt_mesh_locator_build) of as many levels as the tree has, at most
+        JT_MESH_LOCATOR_MAX_DEPTH: a table of 2^21 cells, 16 MB, at 7."""
+        torch = _torch_cuda()
+        m, lib = self.octree_mesh, L.load()
+        desc, dtab = bfs
+        n_entries = int(m.info.n_elem_entries)
+        depth = min(int(m.info.max_tree_depth), m.max_depth, L.JT_MESH_LOCATOR_MAX_DEPTH)
+        S = locator_splits(m.nodes_min[0], m.nodes_max[0], depth) if depth > 0 else None
+        size = int(lib.jt_mesh_locator_bytes(len(dtab), n_entries, depth)) if S is not None else dtab.nbytes
+        block = torch.empty(size, dtype=torch.uint8, device="cuda")
+        block[:dtab.nbytes] = torch.from_numpy(dtab.view(np.uint8).reshape(-1)).cuda()
+        d["desc"], d["dtab"] = torch.from_numpy(desc).cuda(), block
+        f.desc, f.dtab = d["desc"].data_ptr(), block.data_ptr()
+        if S is not None:
+            where = C.c_int32(0)
+            splits = torch.from_numpy(S).cuda()
+            L.check(lib.jt_mesh_locator_build(C.byref(f), n_entries, depth, splits.data_ptr(), C.byref(where),
+                                              L.stream_ptr()))
+            f.locator = where.value
 
     def _device_pairs(self):
         self._device()
