@@ -233,9 +233,9 @@ typedef struct {
  * cells and one table entry; jt_mesh_locator_build compares each centre on
  * the way with `splits` and refuses a tree for which this does not hold.
  *   jt_mesh_locator_bytes: size of the buffer dtab has to point to.
- *   jt_mesh_locator_build: fills it behind dtab's rows.  m: desc, dtab, elems
- *     and tet_geom set; n_entries: length of elems; depth 1..7, at most
- *     max_depth; splits: device (3, 2^depth + 1) float32, ascending, the cell
+ *   jt_mesh_locator_build: fills it behind dtab's rows.  m: desc, dtab, elems,
+ *     tet_box and tet_geom set, each tetrahedron on one list (elems holds
+ *     n_tets entries, as the builds leave it); depth 1..7, at most max_depth; splits: device (3, 2^depth + 1) float32, ascending, the cell
  *     faces of each axis (the outer two are not compared).  *locator_out (host)
  *     receives the value for jt_mesh_field.locator, 0 where the tree does not
  *     split so (the buffer is then not used).  Synchronises the stream. */
@@ -671,9 +671,9 @@ int jt_mark_near_degenerate(float* tet_box, const float* tet_geom, int32_t n_tet
                             void* stream);
 
 /* Locator block of a mesh field (see jt_mesh_field): size, and build. */
-size_t jt_mesh_locator_bytes(int32_t n_nodes, int32_t n_entries, int32_t depth);
-int jt_mesh_locator_build(const jt_mesh_field* m, int32_t n_entries, int32_t depth, const float* splits,
-                          int32_t* locator_out, void* stream);
+size_t jt_mesh_locator_bytes(int32_t n_nodes, int32_t n_tets, int32_t depth);
+int jt_mesh_locator_build(const jt_mesh_field* m, int32_t depth, const float* splits, int32_t* locator_out,
+                          void* stream);
 
 /* Copy the device build's nodes (n_nodes) and node_bounds (n_nodes,6) into
  * caller buffers (device or host; either may be NULL), ordered on `stream`. */

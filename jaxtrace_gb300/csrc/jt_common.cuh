@@ -439,14 +439,31 @@ struct UnrollStagesOf<F, decltype(void(F::kUnrollStages))> {
     static constexpr bool value = F::kUnrollStages;
 };
 
+// Fields that look a query up better from a thread's last hit take a hint
+// word, -1 at first (kHinted, at()); the others ignore it.
+template <class F, class = void>
+struct HintedOf {
+    static constexpr bool value = false;
+};
+template <class F>
+struct HintedOf<F, decltype(void(F::kHinted))> {
+    static constexpr bool value = F::kHinted;
+};
+
+template <class Field>
+__device__ __forceinline__ V3 field_at(const Field& f, const V3& x, const jt_blend& e, int& flags, int& hint) {
+    if constexpr (HintedOf<Field>::value) return f.at(x, e, flags, hint);
+    else return f(x, e, flags);
+}
+
 // RK4 stage st: evaluate at xs, fold k into the weighted sum sm and move xs to
 // the next stage position (rk4.py:82-106).
 template <bool EXACT, class Field>
 __device__ __forceinline__ void rk4_stage(const Field& f, const jt_blend* s, const StepConst& k, int st,
-                                          const V3& x, V3& xs, V3& sm, int& flags) {
+                                          const V3& x, V3& xs, V3& sm, int& flags, int& hint) {
     typedef Ar<EXACT> A;
     const jt_blend e = s[st == 0 ? 0 : (st == 3 ? 2 : 1)];
-    const V3 kk = f(xs, e, flags);
+    const V3 kk = field_at(f, xs, e, flags, hint);
     if (st == 0) {
         sm = kk;
     } else if (st == 3) {
@@ -461,16 +478,16 @@ __device__ __forceinline__ void rk4_stage(const Field& f, const jt_blend* s, con
 // RK2 stage st: evaluate at xs and move xs to the midpoint (rk2.py:283-309).
 template <bool EXACT, class Field>
 __device__ __forceinline__ void rk2_stage(const Field& f, const jt_blend* s, const StepConst& k, int st,
-                                          const V3& x, V3& xs, V3& v, int& flags) {
+                                          const V3& x, V3& xs, V3& v, int& flags, int& hint) {
     typedef Ar<EXACT> A;
     const jt_blend e = s[st];
-    v = f(xs, e, flags);
+    v = field_at(f, xs, e, flags, hint);
     xs = V3{A::axpy(x.x, k.dth, v.x), A::axpy(x.y, k.dth, v.y), A::axpy(x.z, k.dth, v.z)};
 }
 
 template <bool EXACT, int INTEG, bool COMP, class Field>
 __device__ __forceinline__ void integrate(const Field& f, const jt_blend* s, const StepConst& k,
-                                          V3& x, V3& c, int& flags) {
+                                          V3& x, V3& c, int& flags, int& hint) {
     typedef Ar<EXACT> A;
     V3 inc;  // the increment added to x
     if (INTEG == JT_RK4) {
@@ -480,25 +497,25 @@ __device__ __forceinline__ void integrate(const Field& f, const jt_blend* s, con
         V3 sm{0.f, 0.f, 0.f}, xs = x;
         if (UnrollStagesOf<Field>::value) {
 #pragma unroll
-            for (int st = 0; st < 4; ++st) rk4_stage<EXACT>(f, s, k, st, x, xs, sm, flags);
+            for (int st = 0; st < 4; ++st) rk4_stage<EXACT>(f, s, k, st, x, xs, sm, flags, hint);
         } else {
 JT_UNROLL(JT_STAGE_UNROLL)
-            for (int st = 0; st < 4; ++st) rk4_stage<EXACT>(f, s, k, st, x, xs, sm, flags);
+            for (int st = 0; st < 4; ++st) rk4_stage<EXACT>(f, s, k, st, x, xs, sm, flags, hint);
         }
         inc = V3{A::mul(k.dt6, sm.x), A::mul(k.dt6, sm.y), A::mul(k.dt6, sm.z)};
     } else if (INTEG == JT_RK2) {
         V3 xs = x, v{0.f, 0.f, 0.f};
         if (UnrollStagesOf<Field>::value) {
 #pragma unroll
-            for (int st = 0; st < 2; ++st) rk2_stage<EXACT>(f, s, k, st, x, xs, v, flags);
+            for (int st = 0; st < 2; ++st) rk2_stage<EXACT>(f, s, k, st, x, xs, v, flags, hint);
         } else {
 JT_UNROLL(JT_STAGE_UNROLL)
-            for (int st = 0; st < 2; ++st) rk2_stage<EXACT>(f, s, k, st, x, xs, v, flags);
+            for (int st = 0; st < 2; ++st) rk2_stage<EXACT>(f, s, k, st, x, xs, v, flags, hint);
         }
         inc = V3{A::mul(k.dt, v.x), A::mul(k.dt, v.y), A::mul(k.dt, v.z)};
     } else {
         const jt_blend e0 = s[0];
-        V3 v = f(x, e0, flags);
+        V3 v = field_at(f, x, e0, flags, hint);
         inc = V3{A::mul(k.dt, v.x), A::mul(k.dt, v.y), A::mul(k.dt, v.z)};
     }
     if (COMP) {
@@ -568,7 +585,7 @@ __device__ __forceinline__ void track_body(const Field& f, const jt_boundary& B,
         c = V3{cp[0], cp[1], cp[2]};
     }
     const StepConst k{P.dt, P.dt_half, P.dt_sixth};
-    int flags = 0;
+    int flags = 0, hint = -1;
     const int64_t n = P.n_particles;
     // per-particle path length (Trajectory.compute_path_length over rows
     // recorded every step): float32 |x_after - x_before| summed in step order
@@ -581,8 +598,8 @@ __device__ __forceinline__ void track_body(const Field& f, const jt_boundary& B,
     for (int s = P.step_begin; s < P.step_end; ++s) {
         const jt_blend* e = sched + 4 * (int64_t)s;
         const V3 xo = x;
-        if (comp) integrate<EXACT, INTEG, true>(f, e, k, x, c, flags);
-        else integrate<EXACT, INTEG, false>(f, e, k, x, c, flags);
+        if (comp) integrate<EXACT, INTEG, true>(f, e, k, x, c, flags, hint);
+        else integrate<EXACT, INTEG, false>(f, e, k, x, c, flags, hint);
         if constexpr (BK == JT_BK_INLET_XPOS) bc_inlet_xpos<EXACT>(B, I, x.x, x.y, x.z);
         else apply_boundary<EXACT>(B, I, x.x, x.y, x.z);
         if (PATH) {
@@ -600,7 +617,7 @@ __device__ __forceinline__ void track_body(const Field& f, const jt_boundary& B,
                     o[0] = x.x; o[1] = x.y; o[2] = x.z;
                     if (RecordsVelocityOf<Field>::value && P.vel != nullptr) {
                         const jt_blend er = e[3];
-                        V3 v = f(x, er, flags);
+                        V3 v = field_at(f, x, er, flags, hint);
                         float* ov = P.vel + ((int64_t)row * n + id) * 3;
                         ov[0] = v.x; ov[1] = v.y; ov[2] = v.z;
                     }

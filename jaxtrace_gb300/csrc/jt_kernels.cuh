@@ -85,10 +85,10 @@ __global__ void __launch_bounds__(kBlock) k_step(Field f, StageBlends sb, StepCo
         k.dth = __fmul_rn(0.5f, d);
         k.dt6 = __fdiv_rn(d, 6.0f);
     }
-    int flags = 0;
+    int flags = 0, hint = -1;
     V3 x{xin[3 * (int64_t)i], xin[3 * (int64_t)i + 1], xin[3 * (int64_t)i + 2]};
     V3 c{0.f, 0.f, 0.f};
-    integrate<EXACT, INTEG, false>(f, sb.e, k, x, c, flags);
+    integrate<EXACT, INTEG, false>(f, sb.e, k, x, c, flags, hint);
     xout[3 * (int64_t)i] = x.x;
     xout[3 * (int64_t)i + 1] = x.y;
     xout[3 * (int64_t)i + 2] = x.z;

@@ -106,9 +106,8 @@ __device__ __forceinline__ bool tet_bary(const V3& q, const float* tet_box, cons
 //           NaN (nothing is below or above them)
 //   table   8^D {elem_offset, elem_count} of the node that D moves reach, or
 //           {breadth-first node, -1} where the descent goes on below it
-//   slots   64 B per element-list slot: the tetrahedron's tet_geom record,
-//           its first vertex id with the top bit set where the tetrahedron is
-//           well shaped (kWellShaped)
+//   slots   64 B per element-list slot: the tetrahedron's tet_geom record
+//   filters 32 B per element-list slot: the tetrahedron's filter record
 // All offsets are multiples of 64 B from the 64-aligned end of dtab's rows.
 //
 // Why: the evaluation was held by the L1 (93 % busy) on 34 gathers per query,
@@ -122,7 +121,7 @@ __device__ __forceinline__ bool tet_bary(const V3& q, const float* tet_box, cons
 constexpr int32_t kLocatorMagic = 0x4a544c00;  // jt_mesh_field.locator = magic | depth
 
 struct LocatorLayout {
-    size_t header, faces, table, slots, bytes;
+    size_t header, faces, table, slots, filters, bytes;
 };
 
 __host__ __device__ inline LocatorLayout locator_layout(int64_t n_nodes, int64_t n_entries, int depth) {
@@ -132,7 +131,8 @@ __host__ __device__ inline LocatorLayout locator_layout(int64_t n_nodes, int64_t
     o.faces = o.header + 64;
     o.table = al(o.faces + ((size_t)3 << depth) * 8);
     o.slots = al(o.table + ((size_t)8 << (3 * depth)));
-    o.bytes = o.slots + (size_t)n_entries * 64;
+    o.filters = o.slots + (size_t)n_entries * 64;
+    o.bytes = al(o.filters + (size_t)n_entries * 32);
     return o;
 }
 
@@ -141,24 +141,164 @@ __host__ __device__ inline int locator_depth(const jt_mesh_field& F) {
     return (F.locator & ~0xff) == kLocatorMagic && d >= 1 && d <= JT_MESH_LOCATOR_MAX_DEPTH ? d : 0;
 }
 
-// A tetrahedron is well shaped when the cube of its longest edge is at most
-// kWellShaped |det|.  The float32 barycentrics of a query near it are then off
-// by less than 64 * 2^-24 * kWellShaped = 4.9e-4: each numerator is six triple
-// products of components no longer than that edge, three roundings each and
-// five in the sum.  kInside is twice that, so a query whose computed
-// barycentrics are all at least kInside lies inside the tetrahedron, at least
-// 4.9e-4 of the box's extent away from each of its faces, and the box test,
-// whose faces are the vertices' own floats, cannot fail: it is left out.
+// ---------------------------------------------------------------------------
+// Filter records.  A candidate is judged on 32 bytes and nine FMAs instead of
+// its box, its 64-byte geometry and four determinants: words 0-2 hold v0 in
+// float32, words 3-7 the gradients of the barycentrics b1, b2, b3 as nine
+// float16 values (x, y, z of each); the last half-word is the record's slack
+// as a float16, its two low bits the JT_TET_* flags.
+//
+// A query is rejected where a filtered barycentric is below -slack.  That never
+// loses a candidate the full test accepts: such a query lies in the
+// tetrahedron's box, so rounding the gradients to float16 (2^-11 relative, 2^-25
+// absolute) changes no barycentric by more than 2^-11 times the spread, the sum
+// over b1, b2, b3 and the axes of the box's extent times the gradient (and the
+// absolute part), and the full test's own float32 barycentrics are off by at
+// most kShapeError times the shape ratio; slack is above the two together.
+// Where slack would exceed kSlackMost, or the tetrahedron is not well shaped,
+// the gradients are zero: nothing is rejected.
+//
+// A tetrahedron is well shaped when its shape ratio, the cube of its longest
+// edge over |det|, is at most kWellShaped: each numerator of the solve is six
+// triple products of components no longer than that edge, three roundings each
+// and five in the sum, in all less than 64 * 2^-24 times the ratio of the
+// determinant.  A query whose computed barycentrics are all at least kInside
+// then lies inside it, kInsideTrue of its box's extent or more away from each
+// face of the box, and the box test, whose faces are the vertices' own floats,
+// cannot fail.
+//
+// JT_TET_ALONE: well shaped, and no tetrahedron before this one in the list
+// accepts a query whose computed barycentrics here are all at least kInside
+// (checked at build by tets_apart).  Then this tetrahedron is the first hit of
+// every such query, whatever the order they are tried in; one whose filtered
+// barycentrics are all at least slack + kInside is such a query.
+// ---------------------------------------------------------------------------
 constexpr float kWellShaped = 128.0f;
+constexpr float kShapeError = 64.0f / 16777216.0f;
 constexpr float kInside = 1e-3f;
+constexpr float kInsideTrue = kInside - kWellShaped * kShapeError;
+constexpr float kSlackMost = 0.05f;
+enum { JT_TET_SHAPED = 1, JT_TET_ALONE = 2 };
 
-__device__ __forceinline__ bool well_shaped(const float* g12) {
+// Longest edge cubed over |det| of a geometry record; above kWellShaped for a
+// tetrahedron that is not well shaped (a |det| the solve replaces by 1 included).
+__device__ __forceinline__ float shape_ratio(const float* g12, float* longest = nullptr) {
     const V3 a{g12[3], g12[4], g12[5]}, b{g12[6], g12[7], g12[8]}, c{g12[9], g12[10], g12[11]};
     const float det = fabsf(det3<true>(a, b, c));
-    const float la = a.x * a.x + a.y * a.y + a.z * a.z, lb = b.x * b.x + b.y * b.y + b.z * b.z;
-    const float lc = c.x * c.x + c.y * c.y + c.z * c.z;
-    const float l = sqrtf(fmaxf(fmaxf(la, lb), lc));
-    return det >= 1e-10f && l * l * l <= kWellShaped * det;
+    auto len2 = [](float x, float y, float z) { return x * x + y * y + z * z; };
+    const float l = sqrtf(fmaxf(fmaxf(fmaxf(len2(a.x, a.y, a.z), len2(b.x, b.y, b.z)), len2(c.x, c.y, c.z)),
+                                fmaxf(fmaxf(len2(a.x - b.x, a.y - b.y, a.z - b.z), len2(a.x - c.x, a.y - c.y, a.z - c.z)),
+                                      len2(b.x - c.x, b.y - c.y, b.z - c.z))));
+    const float r = l * l * l / det;
+    if (longest != nullptr) *longest = l;
+    return det >= 1e-10f && r <= kWellShaped ? r : 2.0f * kWellShaped;
+}
+
+// Gradients of b1, b2, b3 (the rows of the inverse edge matrix).
+template <class T>
+__device__ __forceinline__ void bary_gradients(const float* g12, T (&g)[3][3]) {
+    const T a[3] = {g12[3], g12[4], g12[5]}, b[3] = {g12[6], g12[7], g12[8]}, c[3] = {g12[9], g12[10], g12[11]};
+    auto cross = [](const T (&u)[3], const T (&v)[3], T (&o)[3]) {
+        o[0] = u[1] * v[2] - u[2] * v[1];
+        o[1] = u[2] * v[0] - u[0] * v[2];
+        o[2] = u[0] * v[1] - u[1] * v[0];
+    };
+    cross(b, c, g[0]);
+    cross(c, a, g[1]);
+    cross(a, b, g[2]);
+    const T det = a[0] * g[0][0] + a[1] * g[0][1] + a[2] * g[0][2];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) g[i][k] = g[i][k] / det;
+}
+
+// Smallest filtered barycentric of q, and the record's slack.
+__device__ __forceinline__ float filter_bary(const V3& q, const uint32_t (&w)[8], float& slack) {
+    const auto h2 = [&w](int i) { return __half22float2(*reinterpret_cast<const __half2*>(&w[i])); };
+    const float px = q.x - __uint_as_float(w[0]), py = q.y - __uint_as_float(w[1]), pz = q.z - __uint_as_float(w[2]);
+    const float2 a = h2(3), b = h2(4), c = h2(5), d = h2(6), e = h2(7);
+    const float b1 = fmaf(px, a.x, fmaf(py, a.y, pz * b.x));
+    const float b2 = fmaf(px, b.y, fmaf(py, c.x, pz * c.y));
+    const float b3 = fmaf(px, d.x, fmaf(py, d.y, pz * e.x));
+    slack = e.y;
+    // minima that let a NaN query through: the full test decides
+    return fminf(fminf(1.0f - (b1 + b2 + b3), b1), fminf(b2, b3));
+}
+
+__device__ __forceinline__ uint32_t filter_flags(const uint32_t (&w)[8]) { return (w[7] >> 16) & 3u; }
+
+// Filter record of a geometry record (g12) with the box b8.
+__device__ __forceinline__ void make_filter(const float* g12, const float* b8, uint32_t flags, uint32_t (&w)[8]) {
+    w[0] = __float_as_uint(g12[0]);
+    w[1] = __float_as_uint(g12[1]);
+    w[2] = __float_as_uint(g12[2]);
+    uint32_t h[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, flags};
+    if (flags & JT_TET_SHAPED) {
+        double g[3][3], spread = 0.0;
+        bary_gradients(g12, g);
+        bool fits = true;
+        for (int i = 0; i < 3; ++i)
+            for (int k = 0; k < 3; ++k) {
+                spread += ((double)b8[4 + k] - (double)b8[k]) * (fabs(g[i][k]) + 0x1p-14);
+                fits &= fabs(g[i][k]) < 65000.0;
+            }
+        const double need = spread * 0x1p-11 + kShapeError * shape_ratio(g12) + 2e-5;
+        if (fits && need <= kSlackMost) {
+            for (int i = 0; i < 9; ++i) h[i] = __half_as_ushort(__double2half(g[i / 3][i % 3]));
+            // one float16 step up and the two low bits cleared again above that
+            h[9] = ((__half_as_ushort(__float2half_ru((float)need)) + 4u) & ~3u) | flags;
+        }
+    }
+    for (int i = 0; i < 5; ++i) w[3 + i] = h[2 * i] | (h[2 * i + 1] << 16);
+}
+
+// How far the well-shaped tetrahedron t (gt), shrunken to barycentrics of
+// kInsideTrue, lies beyond a face of e (ge): the largest such distance over e's
+// faces, in e's barycentrics.  far: the longest offset of t's vertices from v0.
+template <class T>
+__device__ __forceinline__ T beyond_face(const float* ge, const float* gt, T& far) {
+    T g[3][3], hi[4], sum[4];
+    bary_gradients(ge, g);
+    far = 0;
+    for (int j = 0; j < 4; ++j) {  // e's barycentrics at t's vertices
+        T p[3], b[4];
+        for (int k = 0; k < 3; ++k) p[k] = ((T)gt[k] - (T)ge[k]) + (j > 0 ? (T)gt[3 * j + k] : (T)0);
+        far = max(far, abs(p[0]) + abs(p[1]) + abs(p[2]));
+        b[0] = 1;
+        for (int i = 0; i < 3; ++i) {
+            b[i + 1] = p[0] * g[i][0] + p[1] * g[i][1] + p[2] * g[i][2];
+            b[0] -= b[i + 1];
+        }
+        for (int i = 0; i < 4; ++i) {
+            hi[i] = j == 0 ? b[i] : max(hi[i], b[i]);
+            sum[i] = j == 0 ? b[i] : sum[i] + b[i];
+        }
+    }
+    const T m = kInsideTrue;
+    T best = (T)-1e30;
+    for (int i = 0; i < 4; ++i) best = max(best, -(((T)1 - 4 * m) * hi[i] + m * sum[i]));
+    return best;
+}
+
+// Whether tetrahedron e (geometry ge, box be) accepts no query whose computed
+// barycentrics in the well-shaped t (gt, bt) are all at least kInside: boxes
+// apart (a query passes both box tests or neither answer matters), or the
+// shrunken t beyond one face of e by more than e's own test is off.  In float32
+// where that decides it, with 2^-24 P r (16 + 8 r) for the values' own rounding
+// (P: far over e's longest edge; three products a gradient component, divided
+// by a determinant good to 6 r roundings), else in float64.
+__device__ __forceinline__ bool tets_apart(const float* ge, const float* be, const float* gt, const float* bt) {
+    for (int k = 0; k < 3; ++k)
+        if (be[k] > bt[4 + k] || be[4 + k] < bt[k]) return true;
+    float edge, far;
+    const float r = shape_ratio(ge, &edge);
+    if (!(r <= kWellShaped)) return false;
+    const float off = 4e-6f + r * kShapeError;
+    const float d = beyond_face<float>(ge, gt, far);
+    if (d > off + fmaxf(far / edge, 1.0f) * r * (16.0f + 8.0f * r) / 16777216.0f) return true;
+    double far64;
+    return beyond_face<double>(ge, gt, far64) > (double)off;
 }
 
 // The barycentric test of one 64-byte record (tet_bary without the box test).
@@ -216,19 +356,22 @@ struct MeshFieldT {
     // the dependent gather chain is latency-bound: 4 blocks of 256 (64
     // registers, no spills) keep more warps in flight than the default 3
     static constexpr int kMinBlocks = JT_MESH_MIN_BLOCKS;
+    static constexpr bool kHinted = true;
     jt_mesh_field F;
     const char* loc;      // locator block's header, or NULL
     int depth;            // its depth
     uint32_t faces, table, slots;  // offsets from the header
+    const char* filters;
 
     static MeshFieldT create(const jt_mesh_field& d, int) {
-        MeshFieldT m{d, nullptr, locator_depth(d), 0, 0, 0};
+        MeshFieldT m{d, nullptr, locator_depth(d), 0, 0, 0, nullptr};
         if (m.depth > 0) {
-            const LocatorLayout o = locator_layout(d.n_nodes, 0, m.depth);
+            const LocatorLayout o = locator_layout(d.n_nodes, d.n_tets, m.depth);
             m.loc = reinterpret_cast<const char*>(d.dtab) + o.header;
             m.faces = (uint32_t)(o.faces - o.header);
             m.table = (uint32_t)(o.table - o.header);
             m.slots = (uint32_t)(o.slots - o.header);
+            m.filters = m.loc + (o.filters - o.header);
         }
         return m;
     }
@@ -274,26 +417,76 @@ struct MeshFieldT {
         return __ldg(reinterpret_cast<const int2*>(F.dtab) + node);
     }
 
-    // First candidate of the list that holds the query (…optimized.py:309-360),
-    // its P1 value in v; false when there is none.
-    __device__ __forceinline__ bool scan_slots(const V3& q, int2 oc, const jt_blend& e, V3& v) const {
-        const char* rec = loc + slots + (int64_t)oc.x * 64;
-        for (int s = 0; s < oc.y; ++s, rec += 64) {
+    __device__ __forceinline__ bool slot_test(const V3& q, int slot, float4& b, int4& cn) const {
+        const char* rec = loc + slots + (int64_t)slot * 64;
+        uint32_t g0[8], g1[8];
+        ldg256(rec, g0);
+        ldg256(rec + 32, g1);
+        cn = make_int4((int)g1[4], (int)g1[5], (int)g1[6], (int)g1[7]);
+        return slot_bary<EXACT>(q, g0, g1, b);
+    }
+
+    // First candidate of the list oc that holds the query (…optimized.py:309-360).
+    // The filters are read until one is certainly the first hit; the full
+    // test then runs on that candidate, or in list order on those that pass.
+    // hint: the slot of the thread's last certain hit, tried before the list.
+    // Filtering to the end before the full test keeps the warp together: with
+    // the test inside the filter loop 10 lanes of 32 were active and the pass
+    // took 16.8 ms; so, with the hint's record and the next one loaded ahead,
+    // 12.3 ms, against 13.4 ms with the full test on every candidate (1M
+    // particles x 64 steps, 1,572,864 tetrahedra).  Bound by latency and issue
+    // together: L1 71 %, issue 60 %, 15 lanes of 32 active.
+    // w: the hint's filter record, loaded before the leaf was known.
+    __device__ __forceinline__ bool find_slot(const V3& q, int2 oc, int& hint, uint32_t (&w)[8], float4& b,
+                                              int4& cn) const {
+        const int end = oc.x + oc.y;
+        int first = end, s = oc.x;
+        bool certain = false;
+        float slack;
+        if ((unsigned)(hint - oc.x) < (unsigned)oc.y) {
+            certain = filter_bary(q, w, slack) >= slack + kInside;
+            if (certain) first = hint;
+        }
+        if (!certain) {
+            hint = -1;
+            if (s < end) ldg256(filters + (int64_t)s * 32, w);
+            while (s < end) {
+                // the next record is on its way while this one is judged
+                uint32_t nx[8];
+                ldg256(filters + (int64_t)min(s + 1, end - 1) * 32, nx);
+                const float m = filter_bary(q, w, slack);
+                const bool alone = filter_flags(w) & JT_TET_ALONE;
+                if (m >= -slack) {
+                    if (first == end) first = s;
+                    if (alone && m >= slack + kInside) {
+                        certain = true;
+                        first = hint = s;
+                        break;
+                    }
+                }
+                ++s;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) w[k] = nx[k];
+            }
+        }
+        for (s = first; s < end; ++s) {
+            if (!certain && s != first) {
+                ldg256(filters + (int64_t)s * 32, w);
+                if (filter_bary(q, w, slack) < -slack) continue;
+            }
+            const char* rec = loc + slots + (int64_t)s * 64;
             uint32_t g0[8], g1[8];
             ldg256(rec, g0);
             ldg256(rec + 32, g1);
-            float4 b;
             if (!slot_bary<EXACT>(q, g0, g1, b)) continue;
-            const bool inside = (int)g1[4] < 0 && fminf(fminf(b.x, b.y), fminf(b.z, b.w)) >= kInside;
-            if (!inside || (NEAR && !EXACT)) {
-                const int t = __ldg(F.elems + oc.x + s);
+            if (!certain || (NEAR && !EXACT)) {
+                const int t = __ldg(F.elems + s);
                 const float4* bx = reinterpret_cast<const float4*>(F.tet_box) + 2 * (int64_t)t;
                 const float4 mn = __ldg(bx), mx = __ldg(bx + 1);
                 if (!(q.x >= mn.x && q.y >= mn.y && q.z >= mn.z && q.x <= mx.x && q.y <= mx.y && q.z <= mx.z)) continue;
                 if (NEAR && !EXACT && mn.w != 0.0f) b = bary_f64(q, F.tet_geom, t);
             }
-            v = p1_combine<EXACT>(b, node_value((int)(g1[4] & 0x7fffffffu), e), node_value((int)g1[5], e),
-                                  node_value((int)g1[6], e), node_value((int)g1[7], e));
+            cn = make_int4((int)g1[4], (int)g1[5], (int)g1[6], (int)g1[7]);
             return true;
         }
         return false;
@@ -305,6 +498,13 @@ struct MeshFieldT {
     }
 
     __device__ __forceinline__ V3 operator()(const V3& q, const jt_blend& e, int& flags) const {
+        int hint = -1;
+        return at(q, e, flags, hint);
+    }
+
+    // The value at q; hint as find_slot keeps it from one evaluation of a
+    // thread to the next (start with -1).
+    __device__ __forceinline__ V3 at(const V3& q, const jt_blend& e, int& flags, int& hint) const {
         typedef Ar<EXACT> A;
         // fixed-depth descent (…optimized.py:278-302): at most max_depth moves,
         // stopping at a leaf or where the query's octant has no child; then
@@ -312,9 +512,14 @@ struct MeshFieldT {
         // holds the query and whose barycentrics pass the tolerance test
         int2 oc;
         if (loc != nullptr) {
+            uint32_t w[8];
+            ldg256(filters + (int64_t)max(hint, 0) * 32, w);
             oc = locate(q);
-            V3 v;
-            if (scan_slots(q, oc, e, v)) return v;
+            float4 b;
+            int4 cn;
+            if (find_slot(q, oc, hint, w, b, cn))
+                return p1_combine<EXACT>(b, node_value(cn.x, e), node_value(cn.y, e), node_value(cn.z, e),
+                                         node_value(cn.w, e));
         } else {
             if (F.desc != nullptr) {
                 oc = descend(q, 0, 0);
@@ -346,9 +551,14 @@ struct MeshFieldT {
         // of the first candidate; an empty list reads slot -1, which indexes
         // the last tetrahedron
         flags |= JT_STATUS_OCTREE_FALLBACK;
-        int first = oc.y > 0 ? __ldg(F.elems + oc.x) : -1;
-        if (first < 0) first += F.n_tets;
-        const int4 cn = __ldg(reinterpret_cast<const int4*>(F.tet_geom) + 4 * (int64_t)first + 3);
+        int4 cn;
+        if (loc != nullptr && oc.y > 0) {
+            cn = __ldg(reinterpret_cast<const int4*>(loc + slots) + 4 * (int64_t)oc.x + 3);
+        } else {
+            int first = oc.y > 0 ? __ldg(F.elems + oc.x) : -1;
+            if (first < 0) first += F.n_tets;
+            cn = __ldg(reinterpret_cast<const int4*>(F.tet_geom) + 4 * (int64_t)first + 3);
+        }
         const int ids[4] = {cn.x, cn.y, cn.z, cn.w};
         int best = ids[0];
         float bd = 0.0f;

@@ -54,40 +54,72 @@ __global__ void __launch_bounds__(kBlock) k_locator_table(const int4* __restrict
     table[i] = below && depth < max_depth ? make_int2(node, -1) : __ldg(dtab + node);
 }
 
-// A tetrahedron's record into its list slot, 16 B per thread.
-__global__ void __launch_bounds__(kBlock) k_locator_slots(const int32_t* __restrict__ elems,
-                                                          const float* __restrict__ geom, int64_t n,
-                                                          uint4* __restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 4 * n) return;
-    const float* g = geom + 16 * (int64_t)__ldg(elems + (i >> 2));
-    uint4 r = __ldg(reinterpret_cast<const uint4*>(g) + (i & 3));
-    if ((i & 3) == 3 && well_shaped(g)) r.x |= 0x80000000u;
-    out[i] = r;
+// Geometry and filter records of the element lists, one warp per list and one
+// lane per slot.  Lists longer than kAloneMost get no JT_TET_ALONE (the check
+// compares every pair of a list).
+constexpr int kAloneMost = 96;
+
+__global__ void __launch_bounds__(kBlock) k_locator_slots(const int2* __restrict__ dtab, int n_nodes,
+                                                          const int32_t* __restrict__ elems,
+                                                          const float* __restrict__ tet_box,
+                                                          const float* __restrict__ geom, int n_entries,
+                                                          uint4* __restrict__ slots, uint4* __restrict__ filters) {
+    const int node = (blockIdx.x * kBlock + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (node >= n_nodes) return;
+    const int2 oc = __ldg(dtab + node);
+    for (int s = lane; s < oc.y && oc.x + s < n_entries; s += 32) {
+        const int64_t slot = oc.x + s, t = __ldg(elems + slot);
+        const uint4* g4 = reinterpret_cast<const uint4*>(geom) + 4 * t;
+        float g[16], b[8];
+        for (int k = 0; k < 4; ++k) {
+            const uint4 r = __ldg(g4 + k);
+            slots[4 * slot + k] = r;
+            *reinterpret_cast<uint4*>(g + 4 * k) = r;
+        }
+        for (int k = 0; k < 8; ++k) b[k] = __ldg(tet_box + 8 * t + k);
+        uint32_t flags = shape_ratio(g) <= kWellShaped ? JT_TET_SHAPED : 0;
+        if (flags && oc.y <= kAloneMost) {
+            bool alone = true;
+            for (int r = 0; r < s && alone; ++r) {
+                const int64_t o = __ldg(elems + oc.x + r);
+                float ge[12], be[8];
+                for (int k = 0; k < 12; ++k) ge[k] = __ldg(geom + 16 * o + k);
+                for (int k = 0; k < 8; ++k) be[k] = __ldg(tet_box + 8 * o + k);
+                alone = tets_apart(ge, be, g, b);
+            }
+            if (alone) flags |= JT_TET_ALONE;
+        }
+        uint32_t w[8];
+        make_filter(g, b, flags, w);
+        filters[2 * slot] = make_uint4(w[0], w[1], w[2], w[3]);
+        filters[2 * slot + 1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
 }
 
 }  // namespace jt
 
 using namespace jt;
 
-extern "C" size_t jt_mesh_locator_bytes(int32_t n_nodes, int32_t n_entries, int32_t depth) {
-    if (n_nodes < 1 || n_entries < 0 || depth < 1 || depth > JT_MESH_LOCATOR_MAX_DEPTH) return 0;
-    return locator_layout(n_nodes, n_entries, depth).bytes;
+extern "C" size_t jt_mesh_locator_bytes(int32_t n_nodes, int32_t n_tets, int32_t depth) {
+    if (n_nodes < 1 || n_tets < 1 || depth < 1 || depth > JT_MESH_LOCATOR_MAX_DEPTH) return 0;
+    return locator_layout(n_nodes, n_tets, depth).bytes;
 }
 
-extern "C" int jt_mesh_locator_build(const jt_mesh_field* m, int32_t n_entries, int32_t depth, const float* splits,
+extern "C" int jt_mesh_locator_build(const jt_mesh_field* m, int32_t depth, const float* splits,
                                      int32_t* locator_out, void* stream) {
     if (m == nullptr || splits == nullptr || locator_out == nullptr)
         return set_error(JT_ERR_INVALID, "mesh, splits and locator_out are required");
     *locator_out = 0;
-    if (m->desc == nullptr || m->dtab == nullptr || m->elems == nullptr || m->tet_geom == nullptr)
-        return set_error(JT_ERR_INVALID, "the locator needs desc, dtab, elems and tet_geom");
+    if (m->desc == nullptr || m->dtab == nullptr || m->elems == nullptr || m->tet_geom == nullptr ||
+        m->tet_box == nullptr)
+        return set_error(JT_ERR_INVALID, "the locator needs desc, dtab, elems, tet_box and tet_geom");
     if (((uintptr_t)m->dtab & 63u) != 0) return set_error(JT_ERR_INVALID, "dtab must be 64-byte aligned");
-    if (m->n_nodes < 1 || n_entries < 0) return set_error(JT_ERR_INVALID, "n_nodes and n_entries must be positive");
+    if (m->n_nodes < 1 || m->n_tets < 1) return set_error(JT_ERR_INVALID, "n_nodes and n_tets must be positive");
+    if ((int64_t)m->n_nodes > (int64_t)1 << 26) return set_error(JT_ERR_UNSUPPORTED, "too many nodes for a locator");
     if (depth < 1 || depth > JT_MESH_LOCATOR_MAX_DEPTH || depth > m->max_depth)
         return set_error(JT_ERR_INVALID, "locator depth %d must be 1..%d and at most max_depth", depth,
                          JT_MESH_LOCATOR_MAX_DEPTH);
-    const LocatorLayout o = locator_layout(m->n_nodes, n_entries, depth);
+    const LocatorLayout o = locator_layout(m->n_nodes, m->n_tets, depth);
     char* base = reinterpret_cast<char*>(const_cast<int32_t*>(m->dtab));
     float* header = reinterpret_cast<float*>(base + o.header);
     int32_t* mismatch = reinterpret_cast<int32_t*>(header) + 7;
@@ -99,9 +131,9 @@ extern "C" int jt_mesh_locator_build(const jt_mesh_field* m, int32_t n_entries, 
     k_locator_table<<<grid_blocks((int64_t)1 << (3 * depth)), kBlock, 0, s>>>(
         reinterpret_cast<const int4*>(m->desc), reinterpret_cast<const int2*>(m->dtab), splits, depth, m->max_depth,
         reinterpret_cast<int2*>(base + o.table), mismatch);
-    if (n_entries > 0)
-        k_locator_slots<<<grid_blocks(4 * (int64_t)n_entries), kBlock, 0, s>>>(
-            m->elems, m->tet_geom, n_entries, reinterpret_cast<uint4*>(base + o.slots));
+    k_locator_slots<<<grid_blocks(32 * (int64_t)m->n_nodes), kBlock, 0, s>>>(
+        reinterpret_cast<const int2*>(m->dtab), m->n_nodes, m->elems, m->tet_box, m->tet_geom, m->n_tets,
+        reinterpret_cast<uint4*>(base + o.slots), reinterpret_cast<uint4*>(base + o.filters));
     int32_t bad = 0;
     err = cudaGetLastError();
     if (err == cudaSuccess) err = cudaMemcpyAsync(&bad, mismatch, sizeof(bad), cudaMemcpyDeviceToHost, s);

@@ -1132,10 +1132,10 @@ class OctreeFEMTimeSeriesFieldOptimized(_DeviceField):
         torch = _torch_cuda()
         m, lib = self.octree_mesh, L.load()
         desc, dtab = bfs
-        n_entries = int(m.info.n_elem_entries)
         depth = min(int(m.info.max_tree_depth), m.max_depth, L.JT_MESH_LOCATOR_MAX_DEPTH)
-        S = locator_splits(m.nodes_min[0], m.nodes_max[0], depth) if depth > 0 else None
-        size = int(lib.jt_mesh_locator_bytes(len(dtab), n_entries, depth)) if S is not None else dtab.nbytes
+        listed = int(m.info.n_elem_entries) == f.n_tets
+        S = locator_splits(m.nodes_min[0], m.nodes_max[0], depth) if depth > 0 and listed else None
+        size = int(lib.jt_mesh_locator_bytes(len(dtab), f.n_tets, depth)) if S is not None else dtab.nbytes
         block = torch.empty(size, dtype=torch.uint8, device="cuda")
         block[:dtab.nbytes] = torch.from_numpy(dtab.view(np.uint8).reshape(-1)).cuda()
         d["desc"], d["dtab"] = torch.from_numpy(desc).cuda(), block
@@ -1143,7 +1143,7 @@ class OctreeFEMTimeSeriesFieldOptimized(_DeviceField):
         if S is not None:
             where = C.c_int32(0)
             splits = torch.from_numpy(S).cuda()
-            L.check(lib.jt_mesh_locator_build(C.byref(f), n_entries, depth, splits.data_ptr(), C.byref(where),
+            L.check(lib.jt_mesh_locator_build(C.byref(f), depth, splits.data_ptr(), C.byref(where),
                                               L.stream_ptr()))
             f.locator = where.value
 

@@ -94,4 +94,33 @@ def test_locator_refusals():
     lib = L.load()
     assert lib.jt_mesh_locator_bytes(0, 1, 1) == lib.jt_mesh_locator_bytes(1, 1, 8) == 0
     with pytest.raises(ValueError, match="required"):
-        L.check(lib.jt_mesh_locator_build(None, 1, 1, None, None, None))
+        L.check(lib.jt_mesh_locator_build(None, 1, None, None, None))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,integrator", [("pow2", "rk4"), ("odd", "rk4"), ("cut", "rk2"), ("sliver", "rk4"),
+                                             ("offset", "euler"), ("overlap", "rk4")])
+def test_tracks_are_the_descents(name, integrator):
+    """A tracking run, whose evaluations start from the thread's last hit, on
+    conforming meshes and on one whose tetrahedra overlap (each listed twice,
+    the copy moved by a little, so that the first hit is not the only one)."""
+    P, T, leaf, depth = _mesh("pow2" if name == "overlap" else name)
+    if name == "overlap":
+        rng = np.random.default_rng(2)
+        P = np.concatenate([P, P + rng.normal(0, 0.01, P.shape).astype(F32)])
+        T = np.concatenate([T, T + len(P) // 2]).astype(np.int32)[rng.permutation(2 * len(T))]
+    rng = np.random.default_rng(11)
+    lo, hi = P.min(axis=0), P.max(axis=0)
+    D = (rng.normal(size=(3, len(P), 3)) * (hi - lo)).astype(F32)
+    x0 = (lo + (hi - lo) * rng.uniform(size=(5000, 3))).astype(F32)
+    ends = []
+    for locator in (True, False):
+        f = jt.OctreeFEMTimeSeriesFieldOptimized(D, np.array([0, 0.5, 1], F32), P, T, max_elements_per_leaf=leaf,
+                                                 max_depth=depth)
+        f.jt_field()
+        if not locator:
+            f._cmesh.locator = 0
+        bc = jt.mixed_boundary((lo, hi), {"x": "periodic", "y": "reflective", "z": "periodic"})
+        tr = jt.create_tracker(integrator, f, bc, record_final_only=True)
+        ends.append(tr.track_particles(x0, (0.0, 0.6), 61, dt=0.01).positions[-1])
+    assert np.array_equal(ends[0].view(np.uint32), ends[1].view(np.uint32))
