@@ -251,11 +251,29 @@ typedef struct {
     int32_t storage;
     int32_t n_pairs;
     int64_t pair_stride;    /* = n_points                                     */
-    const float* points;    /* device (n_points,4) sorted by cell            */
+    const float* points;    /* device (n_points,4) sorted by cell; with
+                               JT_NEAREST_LISTS set in storage, the candidate
+                               lists of jt_nearest_lists_fill behind them     */
     const int32_t* point_ids; /* device (n_points) original node index of sorted slot */
     const int32_t* cell_start; /* device (cells+1) CSR offsets                 */
     const void* pairs;      /* device value pairs indexed by ORIGINAL node id */
 } jt_nearest_field;
+
+/* Candidate lists of a nearest-node field (no counterpart in the reference;
+ * the node found is the same).  A grid of two cells per cell-list cell and
+ * axis, JT_NEAREST_RIM more on each side, lists per cell every node that can be
+ * the float32 argmin of a query in it, by ascending id; a query outside that
+ * grid, or in a cell whose list would be long (it is empty then), is searched
+ * through the cell list.
+ *   jt_nearest_lists_cells: cells of the grid, 0 where the field gets no lists
+ *     (a single cell-list cell, or more than 2^26 cells).
+ *   jt_nearest_lists_count: fills start (device, cells + 1) with the lists'
+ *     offsets and *total (host) with their length; synchronises the stream.
+ *   jt_nearest_lists_bytes: size of the buffer points has to point to.
+ *   jt_nearest_lists_fill: writes the lists behind f->points, which holds the
+ *     sorted nodes already; f->storage then takes JT_NEAREST_LISTS.          */
+#define JT_NEAREST_LISTS 0x100
+#define JT_NEAREST_RIM 4
 
 /* Tetrahedral mesh field with the hash-grid point location of
  * FEMTimeSeriesField (fields/fem_time_series.py:16-110,
@@ -669,6 +687,12 @@ int jt_octree_build_device(const float* points, int32_t n_points, const int32_t*
  * NULL) receives the number flagged.  Returns after the pass has finished. */
 int jt_mark_near_degenerate(float* tet_box, const float* tet_geom, int32_t n_tets, int32_t* count_out,
                             void* stream);
+
+/* Candidate lists of a nearest-node field (see jt_nearest_field). */
+int64_t jt_nearest_lists_cells(const jt_nearest_field* f);
+int jt_nearest_lists_count(const jt_nearest_field* f, uint32_t* start, int64_t* total, void* stream);
+size_t jt_nearest_lists_bytes(const jt_nearest_field* f, int64_t total);
+int jt_nearest_lists_fill(const jt_nearest_field* f, const uint32_t* start, void* stream);
 
 /* Locator block of a mesh field (see jt_mesh_field): size, and build. */
 size_t jt_mesh_locator_bytes(int32_t n_nodes, int32_t n_tets, int32_t depth);

@@ -54,7 +54,9 @@ static int check_nearest(const jt_nearest_field* q) {
     if (q->pair_stride < q->n_points) return set_error(JT_ERR_INVALID, "pair_stride smaller than n_points");
     if (((uintptr_t)q->pairs & 31u) != 0)
         return set_error(JT_ERR_INVALID, "pairs must be 32-byte aligned (256-bit records)");
-    return check_storage(q->storage);
+    if ((q->storage & JT_NEAREST_LISTS) && ((uintptr_t)q->points & 63u) != 0)
+        return set_error(JT_ERR_INVALID, "candidate lists need points on a 64-byte boundary");
+    return check_storage(q->storage & ~JT_NEAREST_LISTS);
 }
 
 int check_grid_shape(const jt_grid_field& g) {

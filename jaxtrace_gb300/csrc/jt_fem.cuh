@@ -19,8 +19,13 @@ struct FemFieldT {
     static constexpr int kMinBlocks = JT_MESH_MIN_BLOCKS;
     jt_fem_field F;
     float h_min;  // smallest nearest-node cell edge (ring-stop bound)
+    NearestLists lists;
 
-    static FemFieldT create(const jt_fem_field& d, float h) { return FemFieldT{d, h}; }
+    static FemFieldT create(const jt_fem_field& d, float h) {
+        FemFieldT f{d, h, NearestLists{}};
+        if (d.nearest.storage & JT_NEAREST_LISTS) f.lists = nearest_lists(d.nearest);
+        return f;
+    }
 
     __device__ __forceinline__ V3 node_value(int node, const jt_blend& e) const {
         const int64_t base = (int64_t)min(max(e.pair, 0), F.nearest.n_pairs - 1) * F.nearest.pair_stride;
@@ -79,7 +84,8 @@ struct FemFieldT {
         }
         // global nearest node (:311-316)
         flags |= JT_STATUS_OCTREE_FALLBACK;
-        return node_value(nearest_id<EXACT>(F.nearest, h_min, q), e);
+        return node_value(lists.cells > 0 ? nearest_listed<EXACT>(F.nearest, lists, h_min, q)
+                                          : nearest_id<EXACT>(F.nearest, h_min, q), e);
     }
 };
 

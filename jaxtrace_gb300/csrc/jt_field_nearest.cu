@@ -19,14 +19,14 @@ float nearest_min_cell_edge(const jt_nearest_field& f) {
 }
 
 int nearest_track(const jt_nearest_field& f, const jt_boundary& b, const jt_track_params& p, cudaStream_t s) {
-    return NearL::track(f, nearest_min_cell_edge(f), f.storage, b, p, s);
+    return NearL::track(f, nearest_min_cell_edge(f), f.storage & ~JT_NEAREST_LISTS, b, p, s);
 }
 int nearest_step(const jt_nearest_field& f, int arith, const StageBlends& sb, int integ, StepConst k,
                  const float* dtpp, const float* xin, float* xout, int n, int32_t* status, cudaStream_t s) {
-    return NearL::step(f, nearest_min_cell_edge(f), f.storage, arith, sb, integ, k, dtpp, xin, xout, n, status, s);
+    return NearL::step(f, nearest_min_cell_edge(f), f.storage & ~JT_NEAREST_LISTS, arith, sb, integ, k, dtpp, xin, xout, n, status, s);
 }
 int nearest_sample(const jt_nearest_field& f, int arith, const jt_blend& e, const float* pos, float* out,
                    int m, int32_t* status, cudaStream_t s) {
-    return NearL::sample(f, nearest_min_cell_edge(f), f.storage, arith, e, pos, out, m, status, s);
+    return NearL::sample(f, nearest_min_cell_edge(f), f.storage & ~JT_NEAREST_LISTS, arith, e, pos, out, m, status, s);
 }
 }  // namespace jt

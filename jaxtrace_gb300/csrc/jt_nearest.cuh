@@ -1,9 +1,10 @@
 // Scattered-node field: nearest-node sampling of TimeSeriesField
 // (fields/time_series.py:249-259 and :391-412).  The reference takes the
-// argmin over all nodes of the float32 squared distance; here a uniform cell
-// list limits the search to rings of cells around the query, and the ring
-// loop stops once no unvisited cell can hold a point at or below the best
-// squared distance.  Ties go to the lowest node index, as argmin does.
+// argmin over all nodes of the float32 squared distance, the lowest index on
+// ties.  Here a query reads the candidate list of its cell (jt_nearest_lists_fill);
+// outside the lists' grid, and for fields without lists, a uniform cell list
+// limits the search to rings of cells around the query, and the ring loop stops
+// once no unvisited cell can hold a point at or below the best squared distance.
 #pragma once
 
 #include "jt_common.cuh"
@@ -104,16 +105,100 @@ __device__ __forceinline__ int nearest_id(const jt_nearest_field& F, float h_min
     return best_id == 0x7fffffff ? 0 : best_id;
 }
 
+// ---------------------------------------------------------------------------
+// Candidate lists: behind the sorted nodes, 64-byte aligned, the lists' offsets
+// (cells + 1) and then {x, y, z, id} records, ascending ids per list.
+// ---------------------------------------------------------------------------
+struct NearestLists {
+    float org[3], inv[3];  // grid of the lists; a flat axis has one cell
+    int n[3];
+    size_t start, rec;     // offsets from points
+    int64_t cells;         // 0: no lists
+};
+
+__host__ inline NearestLists nearest_lists(const jt_nearest_field& F) {
+    NearestLists g{};
+    float widest = 0.0f;  // the rim of a flat axis is that of the widest live one
+    for (int a = 0; a < 3; ++a)
+        if (F.cells[a] > 1 && F.inv_cell[a] > 0.0f) widest = fmaxf(widest, 0.5f / F.inv_cell[a]);
+    if (!(widest > 0.0f) || !isfinite(widest)) return g;
+    int64_t cells = 1;
+    for (int a = 0; a < 3; ++a) {
+        if (F.inv_cell[a] > 0.0f) {
+            g.n[a] = 2 * F.cells[a] + 2 * JT_NEAREST_RIM;
+            g.inv[a] = 2.0f * F.inv_cell[a];
+            g.org[a] = F.origin[a] - (float)JT_NEAREST_RIM / g.inv[a];
+        } else {
+            g.n[a] = 1;
+            g.inv[a] = 0.5f / ((float)JT_NEAREST_RIM * widest);
+            g.org[a] = F.origin[a] - (float)JT_NEAREST_RIM * widest;
+        }
+        if (!isfinite(g.inv[a]) || !isfinite(g.org[a]) || F.cells[a] > 4096) return g;
+        cells *= g.n[a];
+    }
+    auto al = [](size_t b) { return (b + 63) & ~(size_t)63; };
+    g.start = al((size_t)F.n_points * 16);
+    if (cells > (int64_t)1 << 26) return g;
+    g.cells = cells;
+    g.rec = al(g.start + (size_t)(cells + 1) * 4);
+    return g;
+}
+
+// Cell of q in the lists' grid, -1 outside it and for NaN.
+__device__ __forceinline__ int nearest_list_cell(const NearestLists& g, const V3& q) {
+    const float fx = (q.x - g.org[0]) * g.inv[0], fy = (q.y - g.org[1]) * g.inv[1], fz = (q.z - g.org[2]) * g.inv[2];
+    if (!(fx >= 0.0f && fy >= 0.0f && fz >= 0.0f && fx < (float)g.n[0] && fy < (float)g.n[1] && fz < (float)g.n[2]))
+        return -1;
+    return ((int)fz * g.n[1] + (int)fy) * g.n[0] + (int)fx;
+}
+
+// nearest_id through the candidate lists (g.cells > 0).  One loop of a few
+// contiguous 16-byte records per lane: the rings visit about 27 cells in rows
+// of their own lengths (54 nodes), a ball around a first guess fewer but with
+// per-lane trip counts in three nested loops, which left 5 of 32 lanes active
+// and was slower than the rings.  200,003 particles x 50 RK4 steps over 35,937
+// nodes: 9.3 -> 1.6 ms, 460 warp instructions per evaluation of a warp, 20 of
+// 32 lanes active, bound by the L1 (79 %) on particles in no particular order.
+template <bool EXACT>
+__device__ __forceinline__ int nearest_listed(const jt_nearest_field& F, const NearestLists& g, float h_min,
+                                              const V3& q) {
+    typedef Ar<EXACT> A;
+    const int c = nearest_list_cell(g, q);
+    if (c < 0) return nearest_id<EXACT>(F, h_min, q);
+    const char* base = reinterpret_cast<const char*>(F.points);
+    const uint32_t* st = reinterpret_cast<const uint32_t*>(base + g.start) + c;
+    const uint32_t b = __ldg(st), en = __ldg(st + 1);
+    const float4* rec = reinterpret_cast<const float4*>(base + g.rec);
+    float best = __int_as_float(0x7f800000);
+    int id = 0x7fffffff;
+    for (uint32_t s = b; s < en; ++s) {
+        const float4 p = __ldg(rec + s);
+        const float dx = A::sub(q.x, p.x), dy = A::sub(q.y, p.y), dz = A::sub(q.z, p.z);
+        const float d = A::add(A::add(A::mul(dx, dx), A::mul(dy, dy)), A::mul(dz, dz));
+        if (d < best) {  // ascending ids: the first of a tie stays
+            best = d;
+            id = __float_as_int(p.w);
+        }
+    }
+    return id == 0x7fffffff ? nearest_id<EXACT>(F, h_min, q) : id;
+}
+
 template <bool EXACT, int STORE>
 struct NearestField {
     jt_nearest_field F;
     float h_min;  // smallest cell edge
+    NearestLists lists;
 
-    static NearestField create(const jt_nearest_field& d, float h) { return NearestField{d, h}; }
+    static NearestField create(const jt_nearest_field& d, float h) {
+        NearestField f{d, h, NearestLists{}};
+        if (d.storage & JT_NEAREST_LISTS) f.lists = nearest_lists(d);
+        return f;
+    }
 
     __device__ __forceinline__ V3 operator()(const V3& q, const jt_blend& e, int& flags) const {
         const int64_t base = (int64_t)min(max(e.pair, 0), F.n_pairs - 1) * F.pair_stride;
-        return blend<EXACT, STORE>(load_pair<STORE>(F.pairs, base + nearest_id<EXACT>(F, h_min, q)), e);
+        const int id = lists.cells > 0 ? nearest_listed<EXACT>(F, lists, h_min, q) : nearest_id<EXACT>(F, h_min, q);
+        return blend<EXACT, STORE>(load_pair<STORE>(F.pairs, base + id), e);
     }
 };
 

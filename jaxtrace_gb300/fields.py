@@ -636,8 +636,32 @@ class TimeSeriesField(_DeviceField):
         q.point_ids = self._dev["ids"].data_ptr()
         q.cell_start = self._dev["start"].data_ptr()
         q.pairs = pairs.data_ptr()
+        self._upload_lists(q)
         self._cnear = q
         self._cfield = L.Field(kind=L.JT_FIELD_NEAREST, nearest=C.pointer(q))
+
+    def _upload_lists(self, q):
+        """The candidate lists of the nearest-node search behind the sorted
+        nodes (jt_nearest_lists_fill): about four cells per node and eight
+        16-byte records per cell."""
+        torch = _torch_cuda()
+        lib = L.load()
+        cells = int(lib.jt_nearest_lists_cells(C.byref(q)))
+        if cells == 0:
+            return
+        start = torch.empty(cells + 1, dtype=torch.int32, device="cuda")
+        total = C.c_int64(0)
+        L.check(lib.jt_nearest_lists_count(C.byref(q), start.data_ptr(), C.byref(total), L.stream_ptr()))
+        size = int(lib.jt_nearest_lists_bytes(C.byref(q), total.value))
+        if size > torch.cuda.mem_get_info()[0] // 4:
+            return
+        block = torch.empty(size, dtype=torch.uint8, device="cuda")
+        pts = self._dev["points"]
+        block[:pts.numel() * 4] = pts.view(torch.uint8).reshape(-1)
+        q.points = block.data_ptr()
+        self._dev["points"] = block
+        L.check(lib.jt_nearest_lists_fill(C.byref(q), start.data_ptr(), L.stream_ptr()))
+        q.storage |= L.JT_NEAREST_LISTS
 
     def _device_pairs(self):
         self._device()
