@@ -298,12 +298,22 @@ typedef struct {
      * box, widened slightly, meets the sub-cell.  The element the cell scan
      * would pick holds the query in its box, so it is on the query's
      * sub-cell list, and every element before it there is before it in the
-     * cell list too.  sub_div 0: scan the cell lists. */
+     * cell list too.  sub_div 0: scan the cell lists.  sub_div may carry
+     * JT_FEM_FILTERS: tet_geom then points to jt_fem_filters_bytes bytes whose
+     * part behind the n_tets records jt_fem_filters_build filled. */
     int32_t sub_div;
     int32_t near_degenerate; /* nonzero: tet_box flags some tetrahedra (jt_mark_near_degenerate) */
     const int32_t* sub_start;  /* device (cells*sub_div^3 + 1) CSR offsets     */
     const int32_t* sub_elems;  /* device element ids                          */
 } jt_fem_field;
+
+/* Filter records of a hash-grid field (no counterpart in the reference; the
+ * candidates accepted are the same): 32 bytes per tetrahedron that reject a
+ * candidate without its box and geometry, and mark the tetrahedra that are the
+ * first hit of every query well inside them, which a thread's next query tries
+ * before any list.  jt_fem_filters_build reads the field's lists, boxes and
+ * geometry and writes behind f->tet_geom's n_tets records (32-byte aligned). */
+#define JT_FEM_FILTERS 0x100
 
 #define JT_FIELD_GRID 1
 #define JT_FIELD_MESH 2
@@ -693,6 +703,19 @@ int64_t jt_nearest_lists_cells(const jt_nearest_field* f);
 int jt_nearest_lists_count(const jt_nearest_field* f, uint32_t* start, int64_t* total, void* stream);
 size_t jt_nearest_lists_bytes(const jt_nearest_field* f, int64_t total);
 int jt_nearest_lists_fill(const jt_nearest_field* f, const uint32_t* start, void* stream);
+
+/* Filter records of a hash-grid field (see jt_fem_field). */
+size_t jt_fem_filters_bytes(int32_t n_tets);
+int jt_fem_filters_build(const jt_fem_field* f, void* stream);
+
+/* Sub-cell lists of a hash-grid field with JT_FEM_FILTERS without the entries
+ * whose filter rejects every query of the sub-cell (the first hits stay).
+ * eps: host, the 3 margins the lists were built with.  _count fills start
+ * (device, sub-cells + 1) and *total (host), and synchronises the stream; _fill
+ * writes total entries to elems (device).  start and elems then serve as
+ * sub_start and sub_elems. */
+int jt_fem_prune_count(const jt_fem_field* f, const float* eps, uint32_t* start, int64_t* total, void* stream);
+int jt_fem_prune_fill(const jt_fem_field* f, const float* eps, const uint32_t* start, int32_t* elems, void* stream);
 
 /* Locator block of a mesh field (see jt_mesh_field): size, and build. */
 size_t jt_mesh_locator_bytes(int32_t n_nodes, int32_t n_tets, int32_t depth);

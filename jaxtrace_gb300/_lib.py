@@ -31,6 +31,7 @@ JT_INLET_OFF, JT_INLET_GRID = 0, 1
 JT_ARITH_EXACT, JT_ARITH_COMPENSATED = 0, 1
 JT_MESH_LOCATOR_MAX_DEPTH = 7
 JT_NEAREST_LISTS = 0x100
+JT_FEM_FILTERS = 0x100
 JT_FIELD_GRID, JT_FIELD_MESH, JT_FIELD_NEAREST, JT_FIELD_FEM = 1, 2, 3, 4
 
 STORAGE_CODES = {"f32": JT_STORE_F32, "float32": JT_STORE_F32, "bf16": JT_STORE_BF16,
@@ -187,6 +188,10 @@ def load(build_if_missing: bool = True):
         "jt_nearest_lists_count": (i32, [P(NearestField), vp, P(i64), vp]),
         "jt_nearest_lists_bytes": (C.c_size_t, [P(NearestField), i64]),
         "jt_nearest_lists_fill": (i32, [P(NearestField), vp, vp]),
+        "jt_fem_filters_bytes": (C.c_size_t, [i32]),
+        "jt_fem_filters_build": (i32, [P(FemField), vp]),
+        "jt_fem_prune_count": (i32, [P(FemField), vp, vp, P(i64), vp]),
+        "jt_fem_prune_fill": (i32, [P(FemField), vp, vp, vp, vp]),
         "jt_mesh_locator_bytes": (C.c_size_t, [i32, i32, i32]),
         "jt_mesh_locator_build": (i32, [P(MeshField), i32, vp, P(i32), vp]),
         "jt_pair_log_ratio": (i32, [vp, vp, i32, f32, vp, vp, vp]),

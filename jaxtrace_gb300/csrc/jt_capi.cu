@@ -132,8 +132,10 @@ static int check_field(const jt_field* f) {
             if (h->tet_box == nullptr || h->tet_geom == nullptr || h->cell_start == nullptr ||
                 h->cell_elems == nullptr)
                 return set_error(JT_ERR_INVALID, "FEM field has a NULL array");
-            if (h->sub_div < 0 || h->sub_div > 16 || (h->sub_div > 0 && (h->sub_start == nullptr ||
-                                                                         h->sub_elems == nullptr)))
+            const int div = h->sub_div & ~JT_FEM_FILTERS;
+            if (div != h->sub_div && ((uintptr_t)h->tet_geom & 31u) != 0)
+                return set_error(JT_ERR_INVALID, "filter records need tet_geom on a 32-byte boundary");
+            if (div < 0 || div > 16 || (div > 0 && (h->sub_start == nullptr || h->sub_elems == nullptr)))
                 return set_error(JT_ERR_INVALID, "FEM sub-cell lists: sub_div must be 0..16 with both arrays set");
             return check_nearest(&h->nearest);
         }

@@ -253,52 +253,71 @@ __device__ __forceinline__ void make_filter(const float* g12, const float* b8, u
     for (int i = 0; i < 5; ++i) w[3 + i] = h[2 * i] | (h[2 * i + 1] << 16);
 }
 
-// How far the well-shaped tetrahedron t (gt), shrunken to barycentrics of
-// kInsideTrue, lies beyond a face of e (ge): the largest such distance over e's
-// faces, in e's barycentrics.  far: the longest offset of t's vertices from v0.
-template <class T>
-__device__ __forceinline__ T beyond_face(const float* ge, const float* gt, T& far) {
-    T g[3][3], hi[4], sum[4];
-    bary_gradients(ge, g);
-    far = 0;
-    for (int j = 0; j < 4; ++j) {  // e's barycentrics at t's vertices
-        T p[3], b[4];
-        for (int k = 0; k < 3; ++k) p[k] = ((T)gt[k] - (T)ge[k]) + (j > 0 ? (T)gt[3 * j + k] : (T)0);
-        far = max(far, abs(p[0]) + abs(p[1]) + abs(p[2]));
-        b[0] = 1;
-        for (int i = 0; i < 3; ++i) {
-            b[i + 1] = p[0] * g[i][0] + p[1] * g[i][1] + p[2] * g[i][2];
-            b[0] -= b[i + 1];
-        }
-        for (int i = 0; i < 4; ++i) {
-            hi[i] = j == 0 ? b[i] : max(hi[i], b[i]);
-            sum[i] = j == 0 ? b[i] : sum[i] + b[i];
-        }
-    }
-    const T m = kInsideTrue;
-    T best = (T)-1e30;
-    for (int i = 0; i < 4; ++i) best = max(best, -(((T)1 - 4 * m) * hi[i] + m * sum[i]));
-    return best;
-}
-
 // Whether tetrahedron e (geometry ge, box be) accepts no query whose computed
 // barycentrics in the well-shaped t (gt, bt) are all at least kInside: boxes
-// apart (a query passes both box tests or neither answer matters), or the
-// shrunken t beyond one face of e by more than e's own test is off.  In float32
-// where that decides it, with 2^-24 P r (16 + 8 r) for the values' own rounding
-// (P: far over e's longest edge; three products a gradient component, divided
-// by a determinant good to 6 r roundings), else in float64.
-__device__ __forceinline__ bool tets_apart(const float* ge, const float* be, const float* gt, const float* bt) {
+// apart (a query passes both box tests or neither answer matters), or t shrunken
+// to barycentrics of kInsideTrue disjoint from e grown by what its own test is
+// off (-1e-6 and kShapeError times its shape ratio).  Two disjoint tetrahedra
+// are apart along a face normal of one or the cross product of an edge of each;
+// neighbours that share an edge or a vertex often only along the latter: with
+// the faces of e alone 14 % of a jittered hexahedral split passed.  A
+// projection is off by less than 16 * 2^-24 |n|_1 P, P the largest coordinate
+// beside t's v0, whichever way n itself is rounded.
+__device__ __forceinline__ bool tets_apart(const float (&ge)[12], const float (&be)[8], const float (&gt)[12],
+                                           const float (&bt)[8]) {
     for (int k = 0; k < 3; ++k)
         if (be[k] > bt[4 + k] || be[4 + k] < bt[k]) return true;
-    float edge, far;
-    const float r = shape_ratio(ge, &edge);
+    const float r = shape_ratio(ge);
     if (!(r <= kWellShaped)) return false;
-    const float off = 4e-6f + r * kShapeError;
-    const float d = beyond_face<float>(ge, gt, far);
-    if (d > off + fmaxf(far / edge, 1.0f) * r * (16.0f + 8.0f * r) / 16777216.0f) return true;
-    double far64;
-    return beyond_face<double>(ge, gt, far64) > (double)off;
+    const float grow = 4e-6f + r * kShapeError, m = kInsideTrue;
+    V3 a[4], c[4];  // t shrunken, e grown, beside t's v0
+    float far = 0.0f;
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const float* g = side ? ge : gt;
+        V3* v = side ? c : a;
+        const float w = side ? -grow : m;
+        V3 sum{0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            v[j] = V3{g[0] - gt[0], g[1] - gt[1], g[2] - gt[2]};
+            if (j > 0) v[j] = V3{v[j].x + g[3 * j], v[j].y + g[3 * j + 1], v[j].z + g[3 * j + 2]};
+            sum = V3{sum.x + v[j].x, sum.y + v[j].y, sum.z + v[j].z};
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float f = 1.0f - 4.0f * w;
+            v[j] = V3{f * v[j].x + w * sum.x, f * v[j].y + w * sum.y, f * v[j].z + w * sum.z};
+            far = fmaxf(far, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fabsf(v[j].z)));
+        }
+    }
+    const auto apart_by = [&](const V3& n) {
+        const auto at = [&n](const V3& p) { return n.x * p.x + n.y * p.y + n.z * p.z; };
+        const float a0 = at(a[0]), a1 = at(a[1]), a2 = at(a[2]), a3 = at(a[3]);
+        const float c0 = at(c[0]), c1 = at(c[1]), c2 = at(c[2]), c3 = at(c[3]);
+        const float alo = fminf(fminf(a0, a1), fminf(a2, a3)), ahi = fmaxf(fmaxf(a0, a1), fmaxf(a2, a3));
+        const float clo = fminf(fminf(c0, c1), fminf(c2, c3)), chi = fmaxf(fmaxf(c0, c1), fmaxf(c2, c3));
+        const float tol = 32.0f / 16777216.0f * (fabsf(n.x) + fabsf(n.y) + fabsf(n.z)) * far;
+        return clo - ahi > tol || alo - chi > tol;
+    };
+    const auto apart_along = [&](const V3& u, const V3& v) {
+        return apart_by(V3{u.y * v.z - u.z * v.y, u.z * v.x - u.x * v.z, u.x * v.y - u.y * v.x});
+    };
+    const auto edge = [](const V3* v, int k) {  // 01 02 03 12 13 23
+        const int i = k < 3 ? 0 : (k < 5 ? 1 : 2), j = k < 3 ? k + 1 : (k < 5 ? k - 1 : 3);
+        return V3{v[j].x - v[i].x, v[j].y - v[i].y, v[j].z - v[i].z};
+    };
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const V3* v = side ? a : c;
+        if (apart_along(edge(v, 0), edge(v, 1)) || apart_along(edge(v, 0), edge(v, 2)) ||
+            apart_along(edge(v, 1), edge(v, 2)) || apart_along(edge(v, 3), edge(v, 4)))
+            return true;
+    }
+#pragma unroll
+    for (int k = 0; k < 36; ++k)
+        if (apart_along(edge(a, k / 6), edge(c, k % 6))) return true;
+    return false;
 }
 
 // The barycentric test of one 64-byte record (tet_bary without the box test).
@@ -433,7 +452,7 @@ struct MeshFieldT {
     // Filtering to the end before the full test keeps the warp together: with
     // the test inside the filter loop 10 lanes of 32 were active and the pass
     // took 16.8 ms; so, with the hint's record and the next one loaded ahead,
-    // 12.3 ms, against 13.4 ms with the full test on every candidate (1M
+    // 11.5 ms, against 13.4 ms with the full test on every candidate (1M
     // particles x 64 steps, 1,572,864 tetrahedra).  Bound by latency and issue
     // together: L1 71 %, issue 60 %, 15 lanes of 32 active.
     // w: the hint's filter record, loaded before the leaf was known.

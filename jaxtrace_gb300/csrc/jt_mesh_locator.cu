@@ -70,11 +70,17 @@ __global__ void __launch_bounds__(kBlock) k_locator_slots(const int2* __restrict
     for (int s = lane; s < oc.y && oc.x + s < n_entries; s += 32) {
         const int64_t slot = oc.x + s, t = __ldg(elems + slot);
         const uint4* g4 = reinterpret_cast<const uint4*>(geom) + 4 * t;
-        float g[16], b[8];
+        float g[12], b[8];
+#pragma unroll
         for (int k = 0; k < 4; ++k) {
             const uint4 r = __ldg(g4 + k);
             slots[4 * slot + k] = r;
-            *reinterpret_cast<uint4*>(g + 4 * k) = r;
+            if (k < 3) {
+                g[4 * k] = __uint_as_float(r.x);
+                g[4 * k + 1] = __uint_as_float(r.y);
+                g[4 * k + 2] = __uint_as_float(r.z);
+                g[4 * k + 3] = __uint_as_float(r.w);
+            }
         }
         for (int k = 0; k < 8; ++k) b[k] = __ldg(tet_box + 8 * t + k);
         uint32_t flags = shape_ratio(g) <= kWellShaped ? JT_TET_SHAPED : 0;

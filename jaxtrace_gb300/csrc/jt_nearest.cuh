@@ -152,7 +152,8 @@ __device__ __forceinline__ int nearest_list_cell(const NearestLists& g, const V3
     return ((int)fz * g.n[1] + (int)fy) * g.n[0] + (int)fx;
 }
 
-// nearest_id through the candidate lists (g.cells > 0).  One loop of a few
+// nearest_id through the candidate lists; 0x7fffffff where they have no answer
+// (no lists, a query outside their grid, a cell without a list).  One loop of a few
 // contiguous 16-byte records per lane: the rings visit about 27 cells in rows
 // of their own lengths (54 nodes), a ball around a first guess fewer but with
 // per-lane trip counts in three nested loops, which left 5 of 32 lanes active
@@ -160,11 +161,10 @@ __device__ __forceinline__ int nearest_list_cell(const NearestLists& g, const V3
 // nodes: 9.3 -> 1.6 ms, 460 warp instructions per evaluation of a warp, 20 of
 // 32 lanes active, bound by the L1 (79 %) on particles in no particular order.
 template <bool EXACT>
-__device__ __forceinline__ int nearest_listed(const jt_nearest_field& F, const NearestLists& g, float h_min,
-                                              const V3& q) {
+__device__ __forceinline__ int nearest_listed(const jt_nearest_field& F, const NearestLists& g, const V3& q) {
     typedef Ar<EXACT> A;
-    const int c = nearest_list_cell(g, q);
-    if (c < 0) return nearest_id<EXACT>(F, h_min, q);
+    const int c = g.cells > 0 ? nearest_list_cell(g, q) : -1;
+    if (c < 0) return 0x7fffffff;
     const char* base = reinterpret_cast<const char*>(F.points);
     const uint32_t* st = reinterpret_cast<const uint32_t*>(base + g.start) + c;
     const uint32_t b = __ldg(st), en = __ldg(st + 1);
@@ -180,7 +180,7 @@ __device__ __forceinline__ int nearest_listed(const jt_nearest_field& F, const N
             id = __float_as_int(p.w);
         }
     }
-    return id == 0x7fffffff ? nearest_id<EXACT>(F, h_min, q) : id;
+    return id;
 }
 
 template <bool EXACT, int STORE>
@@ -197,7 +197,8 @@ struct NearestField {
 
     __device__ __forceinline__ V3 operator()(const V3& q, const jt_blend& e, int& flags) const {
         const int64_t base = (int64_t)min(max(e.pair, 0), F.n_pairs - 1) * F.pair_stride;
-        const int id = lists.cells > 0 ? nearest_listed<EXACT>(F, lists, h_min, q) : nearest_id<EXACT>(F, h_min, q);
+        int id = nearest_listed<EXACT>(F, lists, q);
+        if (id == 0x7fffffff) id = nearest_id<EXACT>(F, h_min, q);
         return blend<EXACT, STORE>(load_pair<STORE>(F.pairs, base + id), e);
     }
 };

@@ -931,8 +931,37 @@ class FEMTimeSeriesField(TimeSeriesField):
         f.sub_div = h.sub_div
         f.sub_start, f.sub_elems = d["sub_start"].data_ptr(), d["sub_elems"].data_ptr()
         f.near_degenerate = int(self.n_near_degenerate > 0)
+        self._upload_filters(f, d)
         self._cfem = f
         self._cfield = L.Field(kind=L.JT_FIELD_FEM, fem=C.pointer(f))
+
+    def _upload_filters(self, f, d):
+        """The geometry records with the filter records behind them
+        (jt_fem_filters_build), and the sub-cell lists without the entries
+        those rule out (jt_fem_prune_fill); the mesh keeps its own lists."""
+        torch = _torch_cuda()
+        M = f.n_tets
+        if not 0 < M <= 1 << 26:
+            return
+        block = torch.empty((M * 24,), dtype=torch.float32, device="cuda")
+        block[:M * 16] = d["tet_geom"].reshape(-1)
+        d["tet_geom"] = block
+        f.tet_geom = block.data_ptr()
+        lib = L.load()
+        L.check(lib.jt_fem_filters_build(C.byref(f), L.stream_ptr()))
+        f.sub_div |= L.JT_FEM_FILTERS
+        if self.fem_mesh.sub_div:
+            h = self.fem_mesh
+            eps = np.nextafter(h._eps(h.sub_div, h.cell_size64).astype(F32), F32(np.inf))
+            start = torch.empty_like(d["sub_start"])
+            total = C.c_int64(0)
+            L.check(lib.jt_fem_prune_count(C.byref(f), eps.ctypes.data, start.data_ptr(), C.byref(total),
+                                           L.stream_ptr()))
+            elems = torch.empty(max(total.value, 1), dtype=torch.int32, device="cuda")
+            L.check(lib.jt_fem_prune_fill(C.byref(f), eps.ctypes.data, start.data_ptr(), elems.data_ptr(),
+                                          L.stream_ptr()))
+            d["sub_start"], d["sub_elems"] = start, elems
+            f.sub_start, f.sub_elems = start.data_ptr(), elems.data_ptr()
 
     def __repr__(self) -> str:
         return (f"FEMTimeSeriesField(data={self.data.shape}, times={self.times.shape}, "
