@@ -369,7 +369,7 @@ typedef struct {
                                    set (after a locality sort), else i     */
     int32_t n_ens;
     int32_t block_size;     /* threads per block of the tracking launch:
-                               0 (256), 64, 128 or 256                     */
+                               0 (by n_particles), 64, 128 or 256          */
     float* pos;             /* device (N,3) in/out                            */
     float* comp;            /* device (N,3) Kahan compensation (COMPENSATED) or NULL */
     float* traj;            /* device (rows,N,3) or NULL                      */

@@ -95,6 +95,15 @@ __global__ void __launch_bounds__(kBlock) k_step(Field f, StageBlends sb, StepCo
     report_flags(status, flags);
 }
 
+// Threads per block of a tracking launch whose caller leaves it open: blocks
+// small enough that a few particles reach all 152 SMs, since one thread's chain
+// of evaluations is what such a run waits for.
+inline int track_block(int64_t n) {
+    constexpr int64_t kSms = 152;
+    if (n >= 8 * kSms * kBlock) return kBlock;
+    return n >= 4 * kSms * (kBlock / 2) ? kBlock / 2 : kBlock / 4;
+}
+
 inline unsigned grid_blocks(int64_t n) { return (unsigned)((n + kBlock - 1) / kBlock); }
 
 // Instantiate and launch for a field template FT<EXACT, STORE>.
@@ -110,7 +119,7 @@ struct Launcher {
                                const jt_track_params& P, cudaStream_t st) {
         const FT<EXACT, STORE> f = make<EXACT, STORE>(d, x);
         // block_size was validated to 0, 64, 128 or 256 (<= kBlock, the launch bound)
-        const int bs = P.block_size > 0 ? P.block_size : kBlock;
+        const int bs = P.block_size > 0 ? P.block_size : track_block(P.n_particles);
         const unsigned g = (unsigned)((P.n_particles + bs - 1) / bs);
         const InletFrame I = inlet_frame(B);
         if (P.path != nullptr) return launch_track<EXACT, true>(f, B, I, P, g, bs, st);

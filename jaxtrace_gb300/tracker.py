@@ -49,11 +49,13 @@ class TrackerOptions:
     device_memory_gb   device budget of one trajectory slab
     time_chunk         steps per kernel launch (None: as many as fit)
     sort_every         re-sort particles by cell every k steps for gather
-                       locality (None: from 2^18 particles up, 100 for float32
-                       snapshots and 200 for 16-bit ones; 0: never)
+                       locality (None: on regular grids from 2^18 particles up,
+                       100 for float32 snapshots and 200 for 16-bit ones; on
+                       meshes and scattered nodes 32 from 2^17 up; 0: never)
     sort_bits          cells per axis of that sort, as a power of two
                        (None: 2^7)
-    block_size         threads per block of the tracking kernel (0: 256)
+    block_size         threads per block of the tracking kernel (0: by the
+                       number of particles)
     autotune           pick sort_every / sort_bits / block_size by timing a
                        short sample of the run (``autotune.Autotuner``)
     cuda_graph         capture the whole tracking pass of ``track_ensembles``
@@ -62,6 +64,12 @@ class TrackerOptions:
                        of a chunk of ``stage_chunk`` steps before the tracking
                        launch, so it gathers one time level (the reference's
                        own order of operations; float32 stays bit-identical)
+    stage_min_gain     with ``stage_fields``, how often a float32 'exact' run must
+                       earn back what blending ahead costs (``_stage_gain``);
+                       else the launch gathers snapshot pairs, which gives the
+                       same bits (0: always blend ahead).  The other
+                       arithmetics always do, since their results would differ
+                       in the last bits
     stage_overlap      blend the next chunk's stage fields on a side stream
                        while the current chunk is tracked (a ring twice as deep)
     record_path_length accumulate each particle's path length over every step
@@ -105,6 +113,7 @@ class TrackerOptions:
     autotune: bool = False
     cuda_graph: bool = False
     stage_fields: bool = True
+    stage_min_gain: float = 1.0
     stage_chunk: int = 32
     stage_overlap: bool = True
     row_sink: Optional[Callable[[int, np.ndarray, Optional[np.ndarray], np.ndarray], None]] = None
@@ -348,15 +357,18 @@ class ParticleTracker:
         """Locality re-sort interval: measured best at 100 steps for float32
         snapshots and 200 for 16-bit ones (whose launches are shorter, so the
         sort is a larger share) on the 16.8M-particle precision workload of a
-        regular grid; 32 on tetrahedral meshes, whose lookups lose locality
-        sooner (FEM configuration, octree: 5.28e9 particle-steps/s at 25, 5.27e9
-        at 50, 5.11e9 at 100, 5.15e9 at 10)."""
+        regular grid from 2^18 particles up; 32 on tetrahedral meshes and
+        scattered nodes, whose lookups lose locality sooner, from 2^17 up (64
+        steps, octree, 1M particles: 12.9 ms at 8, 12.5 at 16, 12.3 at 32, 12.4 at
+        64, 18.1 unsorted; 200,000 particles 4.2 ms at 32 and 4.7 unsorted, 60,000
+        2.35 and 2.30; scattered nodes, 200,000 particles 1.68 and 2.09 ms)."""
         se = self.options.sort_every
         if se is None:
-            if n < (1 << 18):
+            from .fields import OctreeFEMTimeSeriesFieldOptimized, TimeSeriesField
+            scattered = isinstance(self._field, (OctreeFEMTimeSeriesFieldOptimized, TimeSeriesField))
+            if n < (1 << (17 if scattered else 18)):
                 return 0
-            from .fields import FEMTimeSeriesField, OctreeFEMTimeSeriesFieldOptimized
-            if isinstance(self._field, (OctreeFEMTimeSeriesFieldOptimized, FEMTimeSeriesField)):
+            if scattered:
                 return 32
             return 100 if self._field._storage == L.JT_STORE_F32 else 200
         return max(int(se), 0)
@@ -367,14 +379,16 @@ class ParticleTracker:
 
     def _engine(self, pos, times, dt, sched_dev=None, status=None, comp=None, ens=None):
         import torch
+        sched = None
         if sched_dev is None:
-            sched_dev = torch.from_numpy(self._schedule(times, dt).view(np.int32).reshape(-1, 8)).cuda()
+            sched = self._schedule(times, dt)
+            sched_dev = torch.from_numpy(sched.view(np.int32).reshape(-1, 8)).cuda()
         if status is None:
             status = torch.zeros(1, dtype=torch.int32, device="cuda")
         if comp is None and self._arith() == L.JT_ARITH_COMPENSATED:
             comp = torch.zeros_like(pos)
         return _Engine(self, pos, len(times) - 1, dt, sched_dev, status, comp, self._sort_every(pos.shape[0]),
-                       ens=ens)
+                       ens=ens, sched=sched)
 
     def _run(self, pos, times, dt, k, compact, n_rows, positions, velocities, rows_out=None) -> int:
         """Advance ``pos`` (device, (N,3)) through all steps, filling rows 1..
@@ -618,7 +632,7 @@ class _Engine:
     """Buffers of one run: positions in slot order, optional Kahan terms, the
     slot -> particle map of the locality sort and the sort workspace."""
 
-    def __init__(self, tracker, pos, n_steps, dt, sched_dev, status, comp, sort_every, ens=None):
+    def __init__(self, tracker, pos, n_steps, dt, sched_dev, status, comp, sort_every, ens=None, sched=None):
         import torch
         self.t, self.out, self.n_steps = tracker, pos, n_steps
         self.status, self.sched = status, sched_dev
@@ -658,12 +672,15 @@ class _Engine:
             if isinstance(tracker._field, StructuredTimeSeriesField):
                 f = tracker._field
                 overlap = bool(tracker.options.stage_overlap)
-                rec_bytes = _stage_node_bytes(f) * (2 if overlap else 1)
-                free = torch.cuda.mem_get_info(pos.device)[0]
-                chunk = _stage_chunk(int(tracker.options.stage_chunk), n_steps, len(f.grid_x) * len(f.grid_y) * len(f.grid_z),
-                                     rec_bytes, free)
-                if chunk > 0:
-                    self.stage = _StageFields(f, sched_dev, n_steps, chunk, overlap=overlap)
+                nodes = len(f.grid_x) * len(f.grid_y) * len(f.grid_z)
+                entries, uid = _stage_entries(sched_dev if sched is None else sched, n_steps, tracker._code)
+                if not (tracker._arith() == L.JT_ARITH_EXACT and
+                        _stage_gain(self.n, n_steps, tracker._code, uid, nodes) < tracker.options.stage_min_gain):
+                    rec_bytes = _stage_node_bytes(f) * (2 if overlap else 1)
+                    free = torch.cuda.mem_get_info(pos.device)[0]
+                    chunk = _stage_chunk(int(tracker.options.stage_chunk), n_steps, nodes, rec_bytes, free)
+                    if chunk > 0:
+                        self.stage = _StageFields(f, entries, uid, pos.device, n_steps, chunk, overlap=overlap)
 
     def _sort(self, first=False):
         src_pos = self.out if first else self.pos
@@ -870,17 +887,13 @@ class _StageFields:
     (an event recorded just before the current launch).
     """
 
-    def __init__(self, field, sched_dev, n_steps: int, chunk: int, overlap: bool = False):
+    def __init__(self, field, entries, uid, dev, n_steps: int, chunk: int, overlap: bool = False):
         import torch
-        from .schedule import BLEND_DTYPE
         self.lib = L.load()
         self.chunk = max(1, min(int(chunk), n_steps))
         self.overlap = bool(overlap)
-        host = np.ascontiguousarray(sched_dev.cpu().numpy()).view(BLEND_DTYPE).reshape(-1)
-        n_ent = 4 * n_steps
-        host = host[:n_ent].copy()
-        every = host.reshape(n_steps, 4)[:, :3].reshape(-1).copy()        # 3 entries per step
-        self.uid = _stage_numbers(every)
+        host, self.uid = entries, uid
+        every = host.reshape(n_steps, 4)[:, :3].reshape(-1)               # 3 entries per step
         first = np.ones(len(every), dtype=bool)
         first[1:] = self.uid[1:] != self.uid[:-1]
         src = every[first]                                                  # one entry per number
@@ -903,7 +916,6 @@ class _StageFields:
             stage[:, k]["form"] = L.JT_BLEND_WEIGHTED
             stage[:, k]["wa"] = scales[uid[:, k]]
             stage[:, k]["wb"] = 0.0
-        dev = sched_dev.device
         self.sched = torch.from_numpy(stage.reshape(-1).view(np.int32).reshape(-1, 8).copy()).to(dev)
         self.src = torch.from_numpy(src.view(np.int32).reshape(-1, 8).copy()).to(dev)
         self.scales = torch.from_numpy(scales).to(dev)
@@ -979,6 +991,32 @@ class _StageFields:
                                              C.c_void_p(None if self.f32 else sc), run, self.out_storage,
                                              C.c_void_p(out), stream))
         return len(runs)
+
+
+def _stage_entries(sched, n_steps: int, integrator: int):
+    """The run's schedule entries on the host (``sched``: a blend array, or its
+    device copy), and the numbers of the stage entries of each step.  An entry
+    that the integrator does not read takes the previous one's content, so no
+    field is blended for it (RK2 reads the first two of a step's three)."""
+    from .schedule import BLEND_DTYPE
+    if not isinstance(sched, np.ndarray):
+        sched = np.ascontiguousarray(sched.cpu().numpy()).view(BLEND_DTYPE).reshape(-1)
+    host = sched[:4 * n_steps].copy()
+    by_step = host.reshape(n_steps, 4)
+    for k in range({L.JT_EULER: 1, L.JT_RK2: 2}.get(integrator, 3), 3):
+        by_step[:, k] = by_step[:, k - 1]
+    return host, _stage_numbers(by_step[:, :3].reshape(-1).copy())
+
+
+def _stage_gain(n: int, n_steps: int, integrator: int, uid, nodes: int) -> float:
+    """What gathering blended fields saves a float32 run over what blending them
+    costs: 10 ps an evaluation against 7.8 ps a node and field (a float32 quad,
+    48 B written) and 0.35 ms for the ring and its launches.  Measured, pairs
+    against blended fields: inlet run at 128^3, 100 RK4 steps, 10,000 particles
+    0.62 and 4.4 ms, 200,000 2.5 and 7.0, 1M 7.9 and 8.9, 2M 15.8 and 12.3;
+    periodic run at 32^3, 30,000 particles 0.65 and 0.97 ms, 100,000 1.5 and 1.1."""
+    evals = {L.JT_EULER: 1, L.JT_RK2: 2}.get(integrator, 4)
+    return 10.0 * evals * n * n_steps / (7.8 * (int(uid[-1]) + 1) * nodes + 3.5e8)
 
 
 def _stage_numbers(entries) -> np.ndarray:
