@@ -360,25 +360,44 @@ __global__ void __launch_bounds__(kKdeThreads) k_kde_grid(jt_kde_params P) {
 
 constexpr int kKbT = 8;  // the 3-D KDE's grid tile edge
 
-// 3-D KDE with register blocking: a block of 64 threads owns an 8^3 tile of
-// grid points and each thread eight of them (two y by four z), so one particle
-// costs a thread three shared loads (its x factor, two y factors in one
-// 64-bit load, four z factors in one 128-bit load), one float32x2 multiply
-// and four float32x2 FMAs (10 % faster than the scalar ones, same bits).  All factors are stored particle-major (32 B per particle and axis):
-// a warp's loads of one particle fall in one 32-byte row per axis, one
-// shared-memory wavefront each.  The tile stays 8^3 so the dilated box of
-// particles each tile visits stays small.  (Four z points per thread of
-// 128, with x and y factors in axis-major rows, took 3 shared loads per 4
-// terms and was 12 % slower, bound by the shared-memory pipe.)
-constexpr int kK8Threads = 64;
-constexpr int kK8Chunk = 240;  // 3 x 240 x 32 B = 22.5 KB: eight blocks (16 warps) per SM
-static_assert(kK8Threads * 8 == kKbT * kKbT * kKbT, "eight grid points per thread");
+// 3-D KDE with register blocking: a block owns an 8^3 tile of grid points, and
+// 16 of its threads the whole tile, 32 points each (two x by four y by four z),
+// so a particle costs a thread three shared loads (64, 128 and 128 bits), four
+// float32x2 multiplies and sixteen float32x2 FMAs.  The block's eight such
+// groups take every eighth particle of a chunk.  Factors are stored
+// particle-major (32 B per particle and axis): a warp's two groups read two
+// adjacent rows, one wavefront a load.  The tile stays 8^3 so that the dilated
+// box of particles each tile visits stays small.
+//
+// Sums run in float32 over at most kKdFlush / 8 = 128 particles a thread, then
+// over the eight groups in pairs, then in float64: an eighth of the float64
+// additions that every thread's own sums would take, which at two lanes a cycle
+// and SM were a third of the time.  3,000,017 particles, 100^3 points: 22.0 ms
+// with eight points a thread (64 threads, float64 sums of their own every 240
+// particles, bound by shared memory), 15.5 ms with 32 in the same box, 10 ms with
+// the ball below; the FMA pipe is 73 % busy.
+//
+// The particles summed are those of the cells that meet the ball of kKdReach
+// radii around the tile: 6 bandwidths for the default radius of 5.  A box of one
+// radius (plus its cells' remainders, up to half a radius) has 1.5 times the
+// volume and drops more: a Gaussian's mass beyond 5 sigma on an axis is 6e-7,
+// beyond a distance of 6 sigma 7e-8.  The estimator cuts its cells to suit.  The
+// rows of cells are listed first, a row a thread and step, and their particles
+// then dealt out in whole chunks: walking the rows one by one cost as much as
+// the finer cells saved.
+constexpr int kKdThreads = 128;
+constexpr int kKdGroups = kKdThreads / 16;
+constexpr int kKdChunk = 256;   // particles in shared memory: 3 x 256 x 32 B = 24 KB
+constexpr int kKdFlush = 1024;  // particles between float64 sums
+constexpr float kKdReach = 1.2f;
+constexpr int kKdRows = 4 * kKdThreads;  // rows of cells listed at a time
+static_assert(kKdGroups * kKbT * kKbT * kKbT <= 3 * kKdChunk * kKbT, "the groups' sums fit the factors' memory");
+static_assert(kKdFlush % kKdChunk == 0, "sums after whole chunks");
 
-__global__ void __launch_bounds__(kK8Threads, 8) k_kde_grid3_blocked(jt_kde_params P) {
-    __shared__ __align__(16) float fx[kK8Chunk][kKbT];
-    __shared__ __align__(16) float fy[kK8Chunk][kKbT];
-    __shared__ __align__(16) float fz[kK8Chunk][kKbT];
+__global__ void __launch_bounds__(kKdThreads, 5) k_kde_grid3_blocked(jt_kde_params P) {
+    __shared__ __align__(16) float fac[3][kKdChunk][kKbT];
     __shared__ float gcoord[3][kKbT];
+    __shared__ uint32_t row_first[kKdRows], row_end[kKdRows], warp_sum[kKdThreads / 32];
     const int t = threadIdx.x;
     const int tiles_a = (P.res[0] + kKbT - 1) / kKbT, tiles_b = (P.res[1] + kKbT - 1) / kKbT;
     const int ta = blockIdx.x % tiles_a, tb = (blockIdx.x / tiles_a) % tiles_b;
@@ -388,86 +407,193 @@ __global__ void __launch_bounds__(kK8Threads, 8) k_kde_grid3_blocked(jt_kde_para
     if (t < 3 * kKbT) {
         const int a = t / kKbT, k = t % kKbT;
         const int na = a == 0 ? n0 : (a == 1 ? n1 : n2), ba = a == 0 ? b0 : (a == 1 ? b1 : b2);
-        gcoord[a][k] = k < na ? __ldg(P.axis[a] + ba + k) : 0.0f;
+        const float* ax = a == 0 ? P.axis[0] : (a == 1 ? P.axis[1] : P.axis[2]);
+        gcoord[a][k] = k < na ? __ldg(ax + ba + k) : 0.0f;
     }
     __syncthreads();
-    // thread -> (pa, y points pb0 and pb0 + 1, z points pc0 .. pc0 + 3); z fastest
-    const int pc0 = 4 * (t & 1);
-    const int pb0 = 2 * ((t >> 1) & 3);
-    const int pa = t >> 3;
+    // thread -> group, x points pa0 and pa0 + 1, y points pb0 .. pb0 + 3, z points pc0 .. pc0 + 3
+    const int grp = t >> 4, pa0 = 2 * ((t >> 2) & 3), pb0 = 4 * ((t >> 1) & 1), pc0 = 4 * (t & 1);
     const jt_sort_grid& g = P.grid;
     const int lim = (1 << g.bits) - 1;
-    const int lo0 = cell_of(gcoord[0][0] - P.radius, g.origin[0], g.inv_cell[0], lim);
-    const int hi0 = cell_of(gcoord[0][n0 - 1] + P.radius, g.origin[0], g.inv_cell[0], lim);
-    const int lo1 = cell_of(gcoord[1][0] - P.radius, g.origin[1], g.inv_cell[1], lim);
-    const int hi1 = cell_of(gcoord[1][n1 - 1] + P.radius, g.origin[1], g.inv_cell[1], lim);
-    const int lo2 = cell_of(gcoord[2][0] - P.radius, g.origin[2], g.inv_cell[2], lim);
-    const int hi2 = cell_of(gcoord[2][n2 - 1] + P.radius, g.origin[2], g.inv_cell[2], lim);
-    double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+    const float x_lo = gcoord[0][0], x_hi = gcoord[0][n0 - 1], y_lo = gcoord[1][0], y_hi = gcoord[1][n1 - 1];
+    const float z_lo = gcoord[2][0], z_hi = gcoord[2][n2 - 1];
+    const float reach = kKdReach * P.radius, far2 = reach * reach;
+    const int lo0 = cell_of(x_lo - reach, g.origin[0], g.inv_cell[0], lim);
+    const int hi0 = cell_of(x_hi + reach, g.origin[0], g.inv_cell[0], lim);
+    const int lo1 = cell_of(y_lo - reach, g.origin[1], g.inv_cell[1], lim);
+    const int hi1 = cell_of(y_hi + reach, g.origin[1], g.inv_cell[1], lim);
+    const int lo2 = cell_of(z_lo - reach, g.origin[2], g.inv_cell[2], lim);
+    const int hi2 = cell_of(z_hi + reach, g.origin[2], g.inv_cell[2], lim);
+    // gap between the tile and cells c of an axis, less 1e-3 of a cell for the
+    // rounding of the particles' cells; the end cells reach to infinity
+    const auto gap = [lim](int c, float org, float inv, float lo, float hi) {
+        if (!(inv > 0.0f)) return 0.0f;
+        const float e = 1.0f / inv;
+        const float below = c < lim ? lo - (org + ((float)c + 1.001f) * e) : 0.0f;
+        const float above = c > 0 ? org + ((float)c - 0.001f) * e - hi : 0.0f;
+        return fmaxf(fmaxf(below, above), 0.0f);
+    };
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    float2 q[2][4][2];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) q[i >> 3][(i >> 1) & 3][i & 1] = make_float2(0.0f, 0.0f);
+    // the groups' float32 sums into float64: thread t owns points 4t .. 4t + 3
+    const auto flush = [&]() {
+        float* red = &fac[0][0][0];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float* o = red + grp * 512 + ((pa0 + i) * kKbT + pb0 + j) * kKbT + pc0;
+                *reinterpret_cast<float4*>(o) = make_float4(q[i][j][0].x, q[i][j][0].y, q[i][j][1].x, q[i][j][1].y);
+                q[i][j][0] = q[i][j][1] = make_float2(0.0f, 0.0f);
+            }
+        __syncthreads();
+        float4 v[kKdGroups];
+#pragma unroll
+        for (int k = 0; k < kKdGroups; ++k) v[k] = *reinterpret_cast<const float4*>(red + k * 512 + 4 * t);
+#pragma unroll
+        for (int w = kKdGroups / 2; w > 0; w >>= 1)
+#pragma unroll
+            for (int k = 0; k < w; ++k)
+                v[k] = make_float4(v[k].x + v[k + w].x, v[k].y + v[k + w].y, v[k].z + v[k + w].z, v[k].w + v[k + w].w);
+        acc[0] += (double)v[0].x;
+        acc[1] += (double)v[0].y;
+        acc[2] += (double)v[0].z;
+        acc[3] += (double)v[0].w;
+        __syncthreads();
+    };
     unsigned long long visits = 0;
-    for (int cz = lo2; cz <= hi2; ++cz)
-        for (int cy = lo1; cy <= hi1; ++cy) {
-            uint32_t b, e;
-            row_range(P.cell_end, lo0, hi0, cy, cz, g.bits, b, e);
-            visits += e - b;
-            for (uint32_t c0 = b; c0 < e; c0 += kK8Chunk) {
-                const int n = (int)min((uint32_t)kK8Chunk, e - c0);
-                for (int j = t; j < n; j += kK8Threads) {
-                    const int64_t pj = c0 + j;
-                    const float px = __ldg(P.particles + 3 * pj), py = __ldg(P.particles + 3 * pj + 1);
-                    const float pz = __ldg(P.particles + 3 * pj + 2);
-                    float ax[kKbT], ay[kKbT], az[kKbT];
+    int summed = 0;  // particles since the last flush
+    const int ny = hi1 - lo1 + 1, rows = ny * (hi2 - lo2 + 1);
+    for (int r0 = 0; r0 < rows; r0 += kKdRows) {
+        // the rows' particle ranges, four rows a thread, and where each ends
+        // among the particles of all of them
+        uint32_t first[4], cnt[4], mine = 0;
 #pragma unroll
-                    for (int q = 0; q < kKbT; ++q) {
-                        const float dx = gcoord[0][q] - px, dy = gcoord[1][q] - py, dz = gcoord[2][q] - pz;
-                        ax[q] = __expf(-dx * dx * P.half_inv_h2);
-                        ay[q] = __expf(-dy * dy * P.half_inv_h2);
-                        az[q] = __expf(-dz * dz * P.half_inv_h2);
-                    }
+        for (int k = 0; k < 4; ++k) {
+            const int r = r0 + 4 * t + k, cz = lo2 + r / ny, cy = lo1 + r % ny;
+            first[k] = cnt[k] = 0;
+            if (r < rows) {
+                const float gz = gap(cz, g.origin[2], g.inv_cell[2], z_lo, z_hi);
+                const float gy = gap(cy, g.origin[1], g.inv_cell[1], y_lo, y_hi);
+                const float rem = far2 - gy * gy - gz * gz;
+                if (rem >= 0.0f) {
+                    const float w = sqrtf(rem) * 1.0001f;
+                    const int xa = max(lo0, cell_of(x_lo - w, g.origin[0], g.inv_cell[0], lim));
+                    const int xb = min(hi0, cell_of(x_hi + w, g.origin[0], g.inv_cell[0], lim));
+                    uint32_t e = 0;
+                    if (xa <= xb) row_range(P.cell_end, xa, xb, cy, cz, g.bits, first[k], e);
+                    cnt[k] = e > first[k] ? e - first[k] : 0u;
+                }
+            }
+            mine += cnt[k];
+        }
+        uint32_t incl = mine;
 #pragma unroll
-                    for (int q = 0; q < kKbT; q += 4) {
-                        *reinterpret_cast<float4*>(&fx[j][q]) = make_float4(ax[q], ax[q + 1], ax[q + 2], ax[q + 3]);
-                        *reinterpret_cast<float4*>(&fy[j][q]) = make_float4(ay[q], ay[q + 1], ay[q + 2], ay[q + 3]);
-                        *reinterpret_cast<float4*>(&fz[j][q]) = make_float4(az[q], az[q + 1], az[q + 2], az[q + 3]);
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((t & 31) >= o) incl += v;
+        }
+        __syncthreads();  // the last batch's rows are read
+        if ((t & 31) == 31) warp_sum[t >> 5] = incl;
+        __syncthreads();
+        uint32_t off = incl - mine, total = 0;
+#pragma unroll
+        for (int w = 0; w < kKdThreads / 32; ++w) {
+            if (w < (t >> 5)) off += warp_sum[w];
+            total += warp_sum[w];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            off += cnt[k];
+            row_first[4 * t + k] = first[k] + cnt[k] - off;  // particle = row_first + its place
+            row_end[4 * t + k] = off;
+        }
+        __syncthreads();
+        visits += total;
+        // chunks of the listed particles, two a thread, the next chunk's
+        // positions on their way while this one is summed
+        float pos[2][3];
+        int row[2] = {0, 0};
+        const auto fetch = [&](uint32_t v0) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const uint32_t v = v0 + t + k * kKdThreads;
+                if (v < total) {
+                    while (row_end[row[k]] <= v) ++row[k];
+                    const float* q3 = P.particles + 3 * (int64_t)(row_first[row[k]] + v);
+                    pos[k][0] = __ldg(q3);
+                    pos[k][1] = __ldg(q3 + 1);
+                    pos[k][2] = __ldg(q3 + 2);
+                }
+            }
+        };
+        fetch(0);
+        for (uint32_t v0 = 0; v0 < total; v0 += kKdChunk) {
+            const int held = (int)min((uint32_t)kKdChunk, total - v0);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int j = t + k * kKdThreads;
+                if (j < held) {
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        float f[kKbT];
+#pragma unroll
+                        for (int i = 0; i < kKbT; ++i) {
+                            const float d = gcoord[a][i] - pos[k][a];
+                            f[i] = __expf(-d * d * P.half_inv_h2);
+                        }
+#pragma unroll
+                        for (int i = 0; i < kKbT; i += 4)
+                            *reinterpret_cast<float4*>(&fac[a][j][i]) = make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]);
                     }
                 }
-                __syncthreads();
-                float p[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-                // float32x2 multiplies and FMAs: each lane rounds as the scalar ones
-                float2 q00 = make_float2(0.f, 0.f), q01 = q00, q10 = q00, q11 = q00;
-#pragma unroll 4
-                for (int j = 0; j < n; ++j) {
-                    const float2 y2 = *reinterpret_cast<const float2*>(&fy[j][pb0]);
-                    const float4 c = *reinterpret_cast<const float4*>(&fz[j][pc0]);
-                    const float2 ab = __fmul2_rn(splat(fx[j][pa]), y2);
-                    const float2 cxy = make_float2(c.x, c.y), czw = make_float2(c.z, c.w);
-                    q00 = __ffma2_rn(splat(ab.x), cxy, q00);
-                    q01 = __ffma2_rn(splat(ab.x), czw, q01);
-                    q10 = __ffma2_rn(splat(ab.y), cxy, q10);
-                    q11 = __ffma2_rn(splat(ab.y), czw, q11);
+            }
+            __syncthreads();
+            fetch(v0 + kKdChunk);
+#pragma unroll 2
+            for (int j = grp; j < held; j += kKdGroups) {
+                const float2 x = *reinterpret_cast<const float2*>(&fac[0][j][pa0]);
+                const float4 y = *reinterpret_cast<const float4*>(&fac[1][j][pb0]);
+                const float4 z = *reinterpret_cast<const float4*>(&fac[2][j][pc0]);
+                const float2 y01 = make_float2(y.x, y.y), y23 = make_float2(y.z, y.w);
+                const float2 z01 = make_float2(z.x, z.y), z23 = make_float2(z.z, z.w);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float2 xx = splat(i ? x.y : x.x);
+                    const float2 p01 = __fmul2_rn(xx, y01), p23 = __fmul2_rn(xx, y23);
+                    q[i][0][0] = __ffma2_rn(splat(p01.x), z01, q[i][0][0]);
+                    q[i][0][1] = __ffma2_rn(splat(p01.x), z23, q[i][0][1]);
+                    q[i][1][0] = __ffma2_rn(splat(p01.y), z01, q[i][1][0]);
+                    q[i][1][1] = __ffma2_rn(splat(p01.y), z23, q[i][1][1]);
+                    q[i][2][0] = __ffma2_rn(splat(p23.x), z01, q[i][2][0]);
+                    q[i][2][1] = __ffma2_rn(splat(p23.x), z23, q[i][2][1]);
+                    q[i][3][0] = __ffma2_rn(splat(p23.y), z01, q[i][3][0]);
+                    q[i][3][1] = __ffma2_rn(splat(p23.y), z23, q[i][3][1]);
                 }
-                p[0][0] = q00.x; p[0][1] = q00.y; p[0][2] = q01.x; p[0][3] = q01.y;
-                p[1][0] = q10.x; p[1][1] = q10.y; p[1][2] = q11.x; p[1][3] = q11.y;
-#pragma unroll
-                for (int r = 0; r < 2; ++r)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) acc[r][k] += (double)p[r][k];
+            }
+            summed += held;
+            if (summed >= kKdFlush) {
+                flush();
+                summed = 0;
+            } else {
                 __syncthreads();
             }
         }
+    }
+    flush();
     if (P.counters != nullptr && t == 0) {
         atomicAdd(P.counters, visits);
         atomicAdd(P.counters + 1, visits * (unsigned long long)(n0 * n1 * n2));
     }
+    const int pa = t >> 4, pb = (t >> 1) & 7, pc = 4 * (t & 1);
+    if (pa < n0 && pb < n1) {
+        const int64_t row = ((int64_t)(b0 + pa) * P.res[1] + (b1 + pb)) * P.res[2] + b2 + pc;
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int pb = pb0 + r;
-        if (pa < n0 && pb < n1) {
-            const int64_t row = ((int64_t)(b0 + pa) * P.res[1] + (b1 + pb)) * P.res[2] + b2 + pc0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (pc0 + k < n2) P.out[row + k] = acc[r][k];
-        }
+        for (int k = 0; k < 4; ++k)
+            if (pc + k < n2) P.out[row + k] = acc[k];
     }
 }
 
@@ -571,7 +697,7 @@ extern "C" int jt_kde_grid(const jt_kde_params* p, void* stream) {
         const int64_t blocks = (int64_t)((p->res[0] + kKbT - 1) / kKbT) * ((p->res[1] + kKbT - 1) / kKbT) *
                                ((p->res[2] + kKbT - 1) / kKbT);
         if (blocks > 0x7fffffff) return set_error(JT_ERR_INVALID, "grid too large");
-        k_kde_grid3_blocked<<<(unsigned)blocks, kK8Threads, 0, st>>>(*p);
+        k_kde_grid3_blocked<<<(unsigned)blocks, kKdThreads, 0, st>>>(*p);
     } else {
         const int T = kTile2;
         const int64_t blocks = (int64_t)((p->res[0] + T - 1) / T) * ((p->res[1] + T - 1) / T);

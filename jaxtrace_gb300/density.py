@@ -135,6 +135,10 @@ def _as_device_f32(positions):
     return torch.from_numpy(np.ascontiguousarray(np.asarray(positions, dtype=F32))).to(_DEV)
 
 
+def _host(a) -> np.ndarray:
+    return a if isinstance(a, np.ndarray) else a.cpu().numpy()
+
+
 def _pad3(P2):
     torch = _torch()
     if P2.shape[1] == 3:
@@ -222,9 +226,9 @@ class KDEEstimator:
             pts2 = self.P[:, [i, j]]
         return pts2.contiguous()
 
-    def _params(self, pts, dims, extent_lo, extent_hi):
+    def _params(self, pts, dims, extent_lo, extent_hi, cell=None):
         radius = float(self.cutoff_sigmas * self.h)
-        cl = CellList(_pad3(pts), extent_lo, extent_hi, max(radius / 2.0, 1e-6), dims)
+        cl = CellList(_pad3(pts), extent_lo, extent_hi, cell if cell else max(radius / 2.0, 1e-6), dims)
         p = L.KdeParams()
         p.dims = dims
         p.n_particles = cl.n
@@ -236,13 +240,21 @@ class KDEEstimator:
         return p, cl
 
     def _grid_sum(self, pts, axes):
-        """sum_j exp(-|g-p_j|^2/2h^2) on the tensor grid of `axes` (x, y[, z])."""
+        """sum_j exp(-|g-p_j|^2/2h^2) on the tensor grid of `axes` (x, y[, z]),
+        a float64 tensor on the device."""
         torch = _torch()
         dims = len(axes)
         ax = [torch.from_numpy(np.ascontiguousarray(a, dtype=F32)).cuda() for a in axes]
         lo = [min(float(pts[:, a].min()), float(axes[a][0])) for a in range(dims)] + [0.0] * (3 - dims)
         hi = [max(float(pts[:, a].max()), float(axes[a][-1])) for a in range(dims)] + [0.0] * (3 - dims)
-        p, cl = self._params(pts, dims, lo, hi)
+        # the 3-D grid kernel cuts a ball out of the cells: about 32 particles
+        # per cell, between a twelfth and half of the radius, hug it
+        cell = None
+        if dims == 3:
+            radius = float(self.cutoff_sigmas * self.h)
+            vol = float(np.prod([max(b - a, 1e-30) for a, b in zip(lo, hi)]))
+            cell = max(min((32.0 * vol / max(int(pts.shape[0]), 1)) ** (1.0 / 3.0), radius / 2.0), radius / 12.0, 1e-6)
+        p, cl = self._params(pts, dims, lo, hi, cell)
         res = [len(a) for a in axes] + [1] * (3 - dims)
         out = torch.empty(int(np.prod(res)), dtype=torch.float64, device="cuda")
         p.res[:] = res
@@ -254,7 +266,7 @@ class KDEEstimator:
             p.counters = counters.data_ptr()
         p.out = out.data_ptr()
         L.check(L.load().jt_kde_grid(C.byref(p), L.stream_ptr()))
-        return out.reshape(res[:dims]).cpu().numpy()
+        return out.reshape(res[:dims])
 
     def _evaluate_points(self, Q, pts):
         torch = _torch()
@@ -311,11 +323,30 @@ class KDEEstimator:
         y = np.linspace(lo[1], hi[1], ny, dtype=np.float32)
         z = np.linspace(lo[2], hi[2], nz, dtype=np.float32)
         X, Y, Z = np.meshgrid(x, y, z, indexing="xy")
-        s = self._reduce(self._grid_sum(self.P, (x, y, z)))   # (nx, ny, nz), all ranks' particles
+        s = self._grid_sum(self.P, (x, y, z))                 # (nx, ny, nz)
+        if self.process_group is None and isinstance(s, _torch().Tensor):
+            return X, Y, Z, self._finish_3d(s, (x, y, z))
+        s = self._reduce(_host(s))                            # all ranks' particles
         D = s.transpose(1, 0, 2) * ((2.0 * math.pi) ** -1.5 / self.N_total)
         if self.normalize:
             D = self._normalise(D, [X, Y, Z], [1, 0, 2])
         return X, Y, Z, D.astype(F32)
+
+    def _finish_3d(self, s, axes):
+        """The sums (nx, ny, nz) on the device to the float32 densities (ny, nx,
+        nz) on the host: evaluate_3d's scale and _normalise in float64, there
+        (2.6 of 5 ms around the kernel for 100^3 points on the host)."""
+        D = s.permute(1, 0, 2) * ((2.0 * math.pi) ** -1.5 / self.N_total)
+        if self.normalize:
+            spans = [float(a.max() - a.min()) for a in axes]
+            cell = 1.0
+            for a, span in zip(axes, spans):
+                cell *= span / max(len(a) - 1, 1)
+            total = (D * cell).sum()
+            D = _torch().where(total > 0, D * (self.N / total), D)
+            avg = self.N / max(spans[0] * spans[1] * spans[2], 1e-12)
+            D = D / max(avg, 1e-12)
+        return D.float().contiguous().cpu().numpy()
 
     def evaluate_2d(self):
         """kde.py:173-186 grid, :205-221 normalisation; returns X, Y, Z of shape (ny, nx)."""
@@ -333,7 +364,7 @@ class KDEEstimator:
         x = np.linspace(lo[0], hi[0], nx, dtype=np.float32)
         y = np.linspace(lo[1], hi[1], ny, dtype=np.float32)
         X, Y = np.meshgrid(x, y, indexing="xy")
-        s = self._reduce(self._grid_sum(pts, (x, y)))         # (nx, ny), all ranks' particles
+        s = self._reduce(_host(self._grid_sum(pts, (x, y))))  # (nx, ny), all ranks' particles
         Z = s.T * ((2.0 * math.pi) ** -1.0 / max(self._count(int(pts.shape[0])), 1))
         if self.normalize:
             Z = self._normalise(Z, [X, Y], [1, 0])

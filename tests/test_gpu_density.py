@@ -70,3 +70,21 @@ def test_sph_and_kde_at_scale_vs_oracle():
     k = KDEEstimator(P, bandwidth=0.03)
     q = rng.random((500, 3)).astype(F32)
     assert np.allclose(k.evaluate(q), OD.kde_mean(q, P, 0.03), rtol=2e-5)
+
+
+@pytest.mark.parametrize("n,res,scale", [(2, (8, 8, 8), 1.0), (3, (1, 9, 17), 1.0), (255, (7, 8, 9), 0.1),
+                                         (1025, (16, 15, 3), 0.3), (40_000, (20, 33, 12), 0.02), (9000, (24, 24, 24), 1.0)])
+@pytest.mark.parametrize("cutoff", [5.0, 6.5])
+def test_kde_3d_grid_tiles_and_row_lists(n, res, scale, cutoff):
+    """Grids that end inside a tile, chunks and row lists that end anywhere (a
+    small bandwidth cuts 2^7 cells per axis, thousands of rows a tile), clumped
+    particles.  Terms dropped lie beyond 1.2 cutoffs: below n exp(-18) in all,
+    which is far below the 2e-5 of the largest sum allowed."""
+    rng = np.random.default_rng(n)
+    P = (0.5 + 0.2 * rng.normal(size=(n, 3)) * np.array([1.0, 0.3, 1.0])).astype(F32)
+    k = KDEEstimator(P, bandwidth=0.1 * scale + 0.01, resolution=res, cutoff_sigmas=cutoff, normalize=False,
+                     bounds=((0.0, 1.0), (-0.2, 1.2), (0.1, 0.9)))
+    X, Y, Z, D = k.evaluate_3d()
+    q = np.stack([X, Y, Z], axis=-1).reshape(-1, 3)
+    ref = OD.kde_mean(q, P, k.h).reshape(D.shape)
+    assert np.allclose(D, ref, rtol=2e-5, atol=2e-5 * ref.max())
