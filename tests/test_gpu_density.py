@@ -88,3 +88,44 @@ def test_kde_3d_grid_tiles_and_row_lists(n, res, scale, cutoff):
     q = np.stack([X, Y, Z], axis=-1).reshape(-1, 3)
     ref = OD.kde_mean(q, P, k.h).reshape(D.shape)
     assert np.allclose(D, ref, rtol=2e-5, atol=2e-5 * ref.max())
+
+
+@pytest.mark.parametrize("kind", ["cubic_spline", "wendland"])
+@pytest.mark.parametrize("dims", ["2d", "3d"])
+@pytest.mark.parametrize("n,h", [(2, 0.5), (3, 0.02), (501, 0.15), (20_000, 0.03), (3000, 1e-3)])
+def test_sph_sums_without_a_support_test(kind, dims, n, h):
+    """Rows that start and end inside a pair of particles, twins (distance 0),
+    few and many candidates, against the float64 sum.  A term is off by a few
+    2^-24 of the kernel's height; 2e-5 of the sum covers one term alone."""
+    rng = np.random.default_rng(n)
+    P = rng.random((n, 3)).astype(F32)
+    P[n // 2:n // 2 + n // 8] = P[:n // 8]
+    m = rng.uniform(0.5, 2.0, n).astype(F32)
+    s = SPHDensityEstimator(P, dimensions=dims, smoothing_length=h, kernel_type=kind, masses=m, normalize=False,
+                            slab_thickness=4.0)
+    q = np.concatenate([P[:300], rng.random((100, 3)).astype(F32)])
+    rho = s.evaluate(q)
+    a, b = (q, P) if dims == "3d" else (q[:, :2], P[:, :2])
+    r = np.sqrt(((a[:, None].astype(np.float64) - b[None]) ** 2).sum(-1)) / np.float64(F32(h))
+    hh = np.float64(F32(h))
+    if kind == "cubic_spline":
+        w = np.where(r <= 1, 1 - 1.5 * r ** 2 + 0.75 * r ** 3, 0.25 * np.clip(2 - r, 0, None) ** 3)
+        w *= 10 / (7 * np.pi * hh ** 2) if dims == "2d" else 1 / (np.pi * hh ** 3)
+    else:
+        w = np.clip(1 - r, 0, None) ** 4 * (1 + 4 * r)
+        w *= 7 / (np.pi * hh ** 2) if dims == "2d" else 21 / (2 * np.pi * hh ** 3)
+    ref = (w * m[None]).sum(1)
+    assert np.allclose(rho, ref, rtol=2e-5, atol=2e-5 * ref.max())
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_sph_particles_that_are_not_finite_stay_where_they_reach(bad):
+    rng = np.random.default_rng(1)
+    P = rng.random((2000, 3)).astype(F32)
+    m = np.ones(2000, F32)
+    q = rng.random((200, 3)).astype(F32)
+    good = SPHDensityEstimator(P, dimensions="3d", smoothing_length=0.05, masses=m, normalize=False).evaluate(q)
+    m[7] = bad
+    rho = SPHDensityEstimator(P, dimensions="3d", smoothing_length=0.05, masses=m, normalize=False).evaluate(q)
+    near = np.linalg.norm(q.astype(np.float64) - P[7], axis=1) < 0.1
+    assert np.allclose(rho[~near], good[~near], rtol=2e-5) and not np.isfinite(rho[near]).any()
