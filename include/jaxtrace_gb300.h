@@ -485,7 +485,8 @@ typedef struct {
     int32_t n_particles;
     int32_t step_begin, step_end;  /* the segment, at most JT_ADJOINT_MAX_SEGMENT steps */
     float dt, dt_half, dt_sixth;   /* as jt_track_params                    */
-    int32_t pad;
+    int32_t stage_storage;         /* JT_STORE_STAGE_F32Q: stage holds quads; any other
+                                      value: JT_STORE_STAGE_F32 node records   */
     const jt_blend* schedule;      /* as jt_track_params.schedule          */
     const float* ckpt;             /* device (N,3): positions at step_begin (forward checkpoint) */
     float* lambda;                 /* device (N,3): dL/dx at step_end on entry, at step_begin on exit */
@@ -498,7 +499,7 @@ typedef struct {
                                       grad is set; zeroed by the call           */
     int64_t work_bytes;
     const float* stage;            /* device float32 stage fields of the segment
-                                      (jt_stage_fields with JT_STORE_STAGE_F32 over its
+                                      (jt_stage_fields with stage_storage over its
                                       3 * steps schedule entries, slot 3*s + k), or NULL to
                                       blend the pair records                     */
 } jt_adjoint_params;

@@ -90,6 +90,9 @@ __device__ __forceinline__ void scatter(const jt_grid_field& F, const Ax3& a, co
     }
 }
 
+// Records per slot of float32 quads (jt_stage_fields): the node count, even.
+__host__ __device__ __forceinline__ int64_t stage_stride(int64_t nodes) { return nodes + (nodes & 1); }
+
 // J^T g at the point with axes a for entry e.  With acc set, the snapshot
 // gradient of this stage, w_c * g per corner node c, is added to acc (one
 // float4 record per node: x, y, z, unused); with `other` set (a second point
@@ -98,14 +101,27 @@ __device__ __forceinline__ void scatter(const jt_grid_field& F, const Ax3& a, co
 // accumulators are folded into the pair-record gradient.
 //
 // STAGE: the blended corner values come from a pre-blended float32 stage
-// field (stage + slot * nodes, one float4 per node) instead of the pair
-// records: half the bytes, no blend arithmetic.
-template <bool STAGE>
+// field (`stage`: its slot) instead of the pair records: no blend arithmetic,
+// and half the bytes (ST_NODES, one float4 per node) or a quarter of the loads
+// (ST_QUADS, yz-quads: one 256-bit and one 128-bit load per x plane).
+enum { ST_PAIRS = 0, ST_NODES = 1, ST_QUADS = 2 };
+
+template <int STAGE>
 __device__ __forceinline__ V3 grid_vjp(const jt_grid_field& F, const Ax3& a, const jt_blend& e, const V3& g,
                                        float4* __restrict__ acc, const Ax3* other, const V3& g_other,
-                                       const float4* __restrict__ stage) {
+                                       const char* __restrict__ stage) {
     float ca = 0.f, cb = 0.f;
-    if (!STAGE) blend_coefs(e, ca, cb);
+    if (STAGE == ST_PAIRS) blend_coefs(e, ca, cb);
+    uint32_t qa[2][8];
+    float4 qz[2];
+    if (STAGE == ST_QUADS) {
+        const int row = a.y.i0 * F.nz + a.z.i0, n0 = a.x.i0 * F.ny * F.nz + row, n1 = a.x.i1 * F.ny * F.nz + row;
+        const char* part_b = stage + stage_stride(F.pair_stride) * 32;
+        ldg256(stage + (int64_t)n0 * 32, qa[0]);
+        ldg256(stage + (int64_t)n1 * 32, qa[1]);
+        qz[0] = __ldg(reinterpret_cast<const float4*>(part_b) + n0);
+        qz[1] = __ldg(reinterpret_cast<const float4*>(part_b) + n1);
+    }
     const int pr = min(max(e.pair, 0), F.n_pairs - 1);
     const int64_t base = (int64_t)pr * F.pair_stride;
     V3 jtg{0.f, 0.f, 0.f};
@@ -118,8 +134,13 @@ __device__ __forceinline__ V3 grid_vjp(const jt_grid_field& F, const Ax3& a, con
         const int64_t node = (int64_t)(i * F.ny + j) * F.nz + k;
         // blended corner value dotted with g
         float vx, vy, vz;
-        if (STAGE) {
-            const float4 v = __ldg(stage + node);
+        if (STAGE == ST_QUADS) {
+            const int i = 2 * by + bz;
+            vx = __uint_as_float(qa[bx][2 * i]);
+            vy = __uint_as_float(qa[bx][2 * i + 1]);
+            vz = i == 0 ? qz[bx].x : (i == 1 ? qz[bx].y : (i == 2 ? qz[bx].z : qz[bx].w));
+        } else if (STAGE == ST_NODES) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(stage) + node);
             vx = v.x; vy = v.y; vz = v.z;
         } else {
             const PairVal pv = load_pair<JT_STORE_F32>(F.pairs, base + node);
@@ -185,7 +206,13 @@ struct StepRec {
 // STAGE: P.stage holds the segment's float32 stage fields (3 per step, slot
 // 3*s + k for stage k of local step s), used for the recompute (bit-identical
 // to blending the pair records) and the vector-Jacobian products.
-template <bool PRE, bool STAGE>
+//
+// The L1 bounds it (85 % with node records, 72 loads of a warp a step; issue
+// 35 %), so quads, which blend three times the bytes, pay: 40 loads, and 15.0 ->
+// 13.2 ms a pass (1M particles x 50 steps at 64^3, both gradients).  What is left
+// (78 %) is the scatter: a lane's 16-byte atomic is a wavefront of its own.  3
+// blocks/SM measured best (2: 13.7, 4: 14.0 ms).
+template <bool PRE, int STAGE>
 __global__ void __launch_bounds__(kBlock, JT_ADJOINT_MIN_BLOCKS)
     k_adjoint_rk4(jt_grid_field F, jt_boundary B, jt_adjoint_params P, float4* __restrict__ acc) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -193,11 +220,13 @@ __global__ void __launch_bounds__(kBlock, JT_ADJOINT_MIN_BLOCKS)
     typedef GridField<true, JT_STORE_F32> Fw;
     const Fw f{F};
     jt_grid_field FS = F;  // the stage fields as a grid descriptor
-    FS.storage = JT_STORE_STAGE_F32;
+    constexpr int kStore = STAGE == ST_QUADS ? JT_STORE_STAGE_F32Q : JT_STORE_STAGE_F32;
+    FS.storage = kStore;
     FS.pairs = P.stage;
     FS.n_pairs = 3 * (P.step_end - P.step_begin);
-    const StageGridField<true, JT_STORE_STAGE_F32> fs = StageGridField<true, JT_STORE_STAGE_F32>::create(FS, 0);
-    const float4* stage4 = reinterpret_cast<const float4*>(P.stage);
+    if (STAGE == ST_QUADS) FS.pair_stride = stage_stride(F.pair_stride);
+    const StageGridField<true, kStore> fs = StageGridField<true, kStore>::create(FS, 0);
+    const int64_t field_bytes = STAGE == ST_QUADS ? FS.pair_stride * 48 : F.pair_stride * 16;
     typedef Ar<true> A;
     const int nseg = P.step_end - P.step_begin;
     const int64_t nodes = F.pair_stride;
@@ -268,9 +297,9 @@ __global__ void __launch_bounds__(kBlock, JT_ADJOINT_MIN_BLOCKS)
         const Ax3 ax4 = axes_of(F, x4);
         const bool join = pend && same_entry(*pend_e, e2) && same_cell(pend_ax, ax4);
         if (pend && !join) scatter(F, pend_ax, pend_g, pend_acc);
-        const float4* s0 = STAGE ? stage4 + (int64_t)(3 * s) * nodes : nullptr;
-        const float4* s1 = STAGE ? s0 + nodes : nullptr;
-        const float4* s2 = STAGE ? s1 + nodes : nullptr;
+        const char* s0 = STAGE ? reinterpret_cast<const char*>(P.stage) + (int64_t)(3 * s) * field_bytes : nullptr;
+        const char* s1 = STAGE ? s0 + field_bytes : nullptr;
+        const char* s2 = STAGE ? s1 + field_bytes : nullptr;
         const V3 d4 = grid_vjp<STAGE>(F, ax4, e2, V3{c6 * lam.x, c6 * lam.y, c6 * lam.z}, join ? pend_acc : a2,
                                       join ? &pend_ax : nullptr, pend_g, s2);                         // k4 = v(x4)
         lx = V3{lx.x + d4.x, lx.y + d4.y, lx.z + d4.z};
@@ -376,12 +405,17 @@ extern "C" int jt_adjoint_rk4(const jt_field* field, const jt_boundary* bc, cons
     bool pre = false;
     for (int a = 0; a < 3; ++a) pre |= bc->axis_kind[a] != JT_BC_PERIODIC && bc->axis_kind[a] != JT_BC_NONE;
     const unsigned gb = grid_blocks(p->n_particles);
-    if (p->stage != nullptr) {
-        if (pre) k_adjoint_rk4<true, true><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
-        else k_adjoint_rk4<false, true><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
+    if (p->stage != nullptr && p->stage_storage == JT_STORE_STAGE_F32Q) {
+        if (((uintptr_t)p->stage & 31u) != 0)
+            return set_error(JT_ERR_INVALID, "stage quads must be 32-byte aligned (256-bit records)");
+        if (pre) k_adjoint_rk4<true, ST_QUADS><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
+        else k_adjoint_rk4<false, ST_QUADS><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
+    } else if (p->stage != nullptr) {
+        if (pre) k_adjoint_rk4<true, ST_NODES><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
+        else k_adjoint_rk4<false, ST_NODES><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
     } else {
-        if (pre) k_adjoint_rk4<true, false><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
-        else k_adjoint_rk4<false, false><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
+        if (pre) k_adjoint_rk4<true, ST_PAIRS><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
+        else k_adjoint_rk4<false, ST_PAIRS><<<gb, kBlock, 0, s>>>(F, *bc, *p, acc);
     }
     int rc = cuda_status(cudaGetLastError(), "adjoint kernel launch");
     if (rc != JT_OK || acc == nullptr) return rc;
