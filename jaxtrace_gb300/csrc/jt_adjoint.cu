@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kBlock, JT_ADJOINT_MIN_BLOCKS)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n_particles) return;
     typedef GridField<true, JT_STORE_F32> Fw;
-    const Fw f{F};
+    const Fw f = Fw::create(F, 0);
     jt_grid_field FS = F;  // the stage fields as a grid descriptor
     constexpr int kStore = STAGE == ST_QUADS ? JT_STORE_STAGE_F32Q : JT_STORE_STAGE_F32;
     FS.storage = kStore;

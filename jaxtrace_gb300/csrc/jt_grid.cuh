@@ -13,15 +13,59 @@
 
 namespace jt {
 
-// Continuous index, cell and weight of one axis (structured.py:289-322).
-// FMA_IDX (fast arithmetic only): the index as one FMA, x * inv_d + nofs with
-// nofs = -x_min * inv_d.
-template <bool EXACT, bool FMA_IDX = false>
-__device__ __forceinline__ void grid_axis(float x, float org, float d, float inv_d, int n, int mode, float vhi,
-                                          int& i0, int& i1, float& w, bool& valid, int& flags, float nofs = 0.0f) {
+// Correctly rounded division by the grid spacings, known before the launch.
+// With z = RN(1/d), q = RN(x z) and r = RN(x - q d), which is exact, RN(q + r z)
+// is RN(x/d) (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", IEEE Trans.
+// Computers 53(8), 2004, after Markstein), provided nothing under- or overflows:
+// spacings within 2^-40 .. 2^40 and |x| within 2^-80 .. 2^60; the others (0
+// among them) take the general division.  Three operations and a share of one
+// guard instead of a general division per axis: 10,000 particles x 100 RK4 steps on
+// pairs 1.08 -> 1.04 ms, 2M on blended fields 12.21 -> 12.11 ms.
+struct ExactDiv {
+    float rinv[3];  // RN(1/spacing)
+    float limit;    // 2^60, or -1 where the spacings do not allow it
+
+    __host__ __device__ static ExactDiv create(const jt_grid_field& F) {
+        ExactDiv e{{0.0f, 0.0f, 0.0f}, 1.152921504606847e18f};
+        for (int a = 0; a < 3; ++a) {
+            const float d = F.spacing[a], m = d < 0.0f ? -d : d;
+            if (!(m >= 9.094947017729282e-13f && m <= 1.099511627776e12f)) e.limit = -1.0f;
+            else e.rinv[a] = 1.0f / d;
+        }
+        return e;
+    }
+
+    __device__ __forceinline__ static float one(float x, float d, float z) {
+        const float q = __fmul_rn(x, z);
+        return __fmaf_rn(__fmaf_rn(-q, d, x), z, q);
+    }
+
+    // (p - origin) / spacing per axis (structured.py:289-291)
+    __device__ __forceinline__ V3 index(const jt_grid_field& F, const V3& p) const {
+        const float x = __fsub_rn(p.x, F.origin[0]), y = __fsub_rn(p.y, F.origin[1]), z = __fsub_rn(p.z, F.origin[2]);
+        const float lo = 8.271806125530277e-25f;  // 2^-80
+        const float least = fminf(fminf(fabsf(x), fabsf(y)), fabsf(z)), most = fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z));
+        if (least >= lo && most <= limit)  // NaN hides from both and stays NaN either way
+            return V3{one(x, F.spacing[0], rinv[0]), one(y, F.spacing[1], rinv[1]), one(z, F.spacing[2], rinv[2])};
+        return V3{__fdiv_rn(x, F.spacing[0]), __fdiv_rn(y, F.spacing[1]), __fdiv_rn(z, F.spacing[2])};
+    }
+};
+
+// Clip that carries NaN, as np_clip: one instruction a bound.  -0 may become +0,
+// which gives the same cell and weight.
+__device__ __forceinline__ float clip_nan(float x, float lo, float hi) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(lo));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(r), "f"(hi));
+    return r;
+}
+
+// Cell and weight of one axis from its continuous index f.
+template <bool EXACT>
+__device__ __forceinline__ void grid_cell(float f, float x, float org, int n, int mode, float vhi, int& i0, int& i1,
+                                          float& w, bool& valid, int& flags) {
     typedef Ar<EXACT> A;
-    // (x - x_min) / dx; the fast modes multiply by the reciprocal
-    float f = EXACT ? __fdiv_rn(__fsub_rn(x, org), d) : (FMA_IDX ? fmaf(x, inv_d, nofs) : (x - org) * inv_d);
     if (mode == JT_GRID_PERIODIC) {
         const int nn = n > 1 ? n : 1;
         f = np_mod(f, (float)nn);          // np.mod(fx, max(Nx,1))
@@ -42,7 +86,7 @@ __device__ __forceinline__ void grid_axis(float x, float org, float d, float inv
         // np.clip(fx, 0, max(Nx-1,0)); the fast modes clip with min/max, which
         // send NaN to cell 0 instead of carrying it in the weight (the
         // particle's position stays NaN either way)
-        f = EXACT ? np_clip(f, 0.0f, hi) : fminf(fmaxf(f, 0.0f), hi);
+        f = EXACT ? clip_nan(f, 0.0f, hi) : fminf(fmaxf(f, 0.0f), hi);
         const float fl = floorf(f);
         // fl is an integer in [0, n-1] (n <= 2^24, so n-1 is exact), or NaN,
         // which converts to 0: the cell is always in range
@@ -51,6 +95,17 @@ __device__ __forceinline__ void grid_axis(float x, float org, float d, float inv
         i0 = i;
         i1 = (i + 1 > n - 1) ? (n - 1) : i + 1;  // np.clip(i0+1, 0, max(Nx-1,0))
     }
+}
+
+// Continuous index, cell and weight of one axis (structured.py:289-322).
+// FMA_IDX (fast arithmetic only): the index as one FMA, x * inv_d + nofs with
+// nofs = -x_min * inv_d.
+template <bool EXACT, bool FMA_IDX = false>
+__device__ __forceinline__ void grid_axis(float x, float org, float d, float inv_d, int n, int mode, float vhi,
+                                          int& i0, int& i1, float& w, bool& valid, int& flags, float nofs = 0.0f) {
+    // (x - x_min) / dx; the fast modes multiply by the reciprocal
+    const float f = EXACT ? __fdiv_rn(__fsub_rn(x, org), d) : (FMA_IDX ? fmaf(x, inv_d, nofs) : (x - org) * inv_d);
+    grid_cell<EXACT>(f, x, org, n, mode, vhi, i0, i1, w, valid, flags);
 }
 
 // A corner value after the time blend: (x,y) packed, z apart.
@@ -126,20 +181,28 @@ __device__ __forceinline__ float2 h2f2(uint32_t w) { return __half22float2(*rein
 template <bool EXACT, int STORE>
 struct GridField {
     jt_grid_field F;
+    ExactDiv div;
 
-    static GridField create(const jt_grid_field& d, int) { return GridField{d}; }
+    __host__ __device__ static GridField create(const jt_grid_field& d, int) { return GridField{d, ExactDiv::create(d)}; }
 
     __device__ __forceinline__ V3 operator()(const V3& p, const jt_blend& e, int& flags) const {
         typedef Ar<EXACT> A;
         int i0, i1, j0, j1, k0, k1;
         float wx, wy, wz;
         bool vx, vy, vz;
-        grid_axis<EXACT>(p.x, F.origin[0], F.spacing[0], F.inv_spacing[0], F.nx, F.bounds_mode, F.valid_hi[0], i0,
-                         i1, wx, vx, flags);
-        grid_axis<EXACT>(p.y, F.origin[1], F.spacing[1], F.inv_spacing[1], F.ny, F.bounds_mode, F.valid_hi[1], j0,
-                         j1, wy, vy, flags);
-        grid_axis<EXACT>(p.z, F.origin[2], F.spacing[2], F.inv_spacing[2], F.nz, F.bounds_mode, F.valid_hi[2], k0,
-                         k1, wz, vz, flags);
+        if (EXACT) {
+            const V3 f = div.index(F, p);
+            grid_cell<EXACT>(f.x, p.x, F.origin[0], F.nx, F.bounds_mode, F.valid_hi[0], i0, i1, wx, vx, flags);
+            grid_cell<EXACT>(f.y, p.y, F.origin[1], F.ny, F.bounds_mode, F.valid_hi[1], j0, j1, wy, vy, flags);
+            grid_cell<EXACT>(f.z, p.z, F.origin[2], F.nz, F.bounds_mode, F.valid_hi[2], k0, k1, wz, vz, flags);
+        } else {
+            grid_axis<EXACT>(p.x, F.origin[0], F.spacing[0], F.inv_spacing[0], F.nx, F.bounds_mode, F.valid_hi[0], i0,
+                             i1, wx, vx, flags);
+            grid_axis<EXACT>(p.y, F.origin[1], F.spacing[1], F.inv_spacing[1], F.ny, F.bounds_mode, F.valid_hi[1], j0,
+                             j1, wy, vy, flags);
+            grid_axis<EXACT>(p.z, F.origin[2], F.spacing[2], F.inv_spacing[2], F.nz, F.bounds_mode, F.valid_hi[2], k0,
+                             k1, wz, vz, flags);
+        }
 
         const int pr = min(max(e.pair, 0), F.n_pairs - 1);
         const int64_t base = (int64_t)pr * F.pair_stride;
@@ -262,9 +325,10 @@ struct StageGridField {
     jt_grid_field F;
     float nofs[3];  // -origin * inv_spacing per axis (fast arithmetic)
     int sx;         // node stride of the x axis, ny * nz
+    ExactDiv div;
 
     __host__ __device__ static StageGridField create(const jt_grid_field& d, int) {
-        StageGridField s{d, {0.0f, 0.0f, 0.0f}, d.ny * d.nz};
+        StageGridField s{d, {0.0f, 0.0f, 0.0f}, d.ny * d.nz, ExactDiv::create(d)};
         for (int a = 0; a < 3; ++a) s.nofs[a] = -d.origin[a] * d.inv_spacing[a];
         return s;
     }
@@ -274,12 +338,19 @@ struct StageGridField {
         int i0, i1, j0, j1, k0, k1;
         float wx, wy, wz;
         bool vx, vy, vz;
-        grid_axis<EXACT, !EXACT>(p.x, F.origin[0], F.spacing[0], F.inv_spacing[0], F.nx, mode, F.valid_hi[0], i0,
-                                 i1, wx, vx, flags, nofs[0]);
-        grid_axis<EXACT, !EXACT>(p.y, F.origin[1], F.spacing[1], F.inv_spacing[1], F.ny, mode, F.valid_hi[1], j0,
-                                 j1, wy, vy, flags, nofs[1]);
-        grid_axis<EXACT, !EXACT>(p.z, F.origin[2], F.spacing[2], F.inv_spacing[2], F.nz, mode, F.valid_hi[2], k0,
-                                 k1, wz, vz, flags, nofs[2]);
+        if (EXACT) {
+            const V3 f = div.index(F, p);
+            grid_cell<EXACT>(f.x, p.x, F.origin[0], F.nx, mode, F.valid_hi[0], i0, i1, wx, vx, flags);
+            grid_cell<EXACT>(f.y, p.y, F.origin[1], F.ny, mode, F.valid_hi[1], j0, j1, wy, vy, flags);
+            grid_cell<EXACT>(f.z, p.z, F.origin[2], F.nz, mode, F.valid_hi[2], k0, k1, wz, vz, flags);
+        } else {
+            grid_axis<EXACT, true>(p.x, F.origin[0], F.spacing[0], F.inv_spacing[0], F.nx, mode, F.valid_hi[0], i0,
+                                   i1, wx, vx, flags, nofs[0]);
+            grid_axis<EXACT, true>(p.y, F.origin[1], F.spacing[1], F.inv_spacing[1], F.ny, mode, F.valid_hi[1], j0,
+                                   j1, wy, vy, flags, nofs[1]);
+            grid_axis<EXACT, true>(p.z, F.origin[2], F.spacing[2], F.inv_spacing[2], F.nz, mode, F.valid_hi[2], k0,
+                                   k1, wz, vz, flags, nofs[2]);
+        }
         const int slot = min(max(e.pair, 0), F.n_pairs - 1);
         const int64_t base = (int64_t)slot * F.pair_stride;
         // 32-bit node offsets within the slot (fewer than 2^31 nodes), scaled
