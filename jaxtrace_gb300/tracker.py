@@ -49,9 +49,9 @@ class TrackerOptions:
     device_memory_gb   device budget of one trajectory slab
     time_chunk         steps per kernel launch (None: as many as fit)
     sort_every         re-sort particles by cell every k steps for gather
-                       locality (None: on regular grids from 2^18 particles up,
-                       100 for float32 snapshots and 200 for 16-bit ones; on
-                       meshes and scattered nodes 32 from 2^17 up; 0: never)
+                       locality (None: on regular grids 50 from 2^18 particles
+                       up, on meshes and scattered nodes 32 from 2^17 up; 0:
+                       never)
     sort_bits          cells per axis of that sort, as a power of two
                        (None: 2^7)
     block_size         threads per block of the tracking kernel (0: by the
@@ -354,10 +354,10 @@ class ParticleTracker:
         return p
 
     def _sort_every(self, n: int) -> int:
-        """Locality re-sort interval: measured best at 100 steps for float32
-        snapshots and 200 for 16-bit ones (whose launches are shorter, so the
-        sort is a larger share) on the 16.8M-particle precision workload of a
-        regular grid from 2^18 particles up; 32 on tetrahedral meshes and
+        """Locality re-sort interval: 50 steps on a regular grid from 2^18
+        particles up (inlet run at 128^3: float32, 2M particles x 400 steps 42.0
+        ms at 50, 42.2 at 34, 42.4 at 100, 43.9 at 200; bfloat16, 16.8M x 200 68.3
+        at 50, 69.2 at 34, 68.7 at 100, 70.9 at 200); 32 on tetrahedral meshes and
         scattered nodes, whose lookups lose locality sooner, from 2^17 up (64
         steps, octree, 1M particles: 12.9 ms at 8, 12.5 at 16, 12.3 at 32, 12.4 at
         64, 18.1 unsorted; 200,000 particles 4.2 ms at 32 and 4.7 unsorted, 60,000
@@ -370,7 +370,7 @@ class ParticleTracker:
                 return 0
             if scattered:
                 return 32
-            return 100 if self._field._storage == L.JT_STORE_F32 else 200
+            return 50
         return max(int(se), 0)
 
     def _sort_bits(self) -> int:
@@ -385,10 +385,11 @@ class ParticleTracker:
             sched_dev = torch.from_numpy(sched.view(np.int32).reshape(-1, 8)).cuda()
         if status is None:
             status = torch.zeros(1, dtype=torch.int32, device="cuda")
+        comp_zero = comp is None
         if comp is None and self._arith() == L.JT_ARITH_COMPENSATED:
             comp = torch.zeros_like(pos)
         return _Engine(self, pos, len(times) - 1, dt, sched_dev, status, comp, self._sort_every(pos.shape[0]),
-                       ens=ens, sched=sched)
+                       ens=ens, sched=sched, comp_zero=comp_zero)
 
     def _run(self, pos, times, dt, k, compact, n_rows, positions, velocities, rows_out=None) -> int:
         """Advance ``pos`` (device, (N,3)) through all steps, filling rows 1..
@@ -632,7 +633,8 @@ class _Engine:
     """Buffers of one run: positions in slot order, optional Kahan terms, the
     slot -> particle map of the locality sort and the sort workspace."""
 
-    def __init__(self, tracker, pos, n_steps, dt, sched_dev, status, comp, sort_every, ens=None, sched=None):
+    def __init__(self, tracker, pos, n_steps, dt, sched_dev, status, comp, sort_every, ens=None, sched=None,
+                 comp_zero=False):
         import torch
         self.t, self.out, self.n_steps = tracker, pos, n_steps
         self.status, self.sched = status, sched_dev
@@ -656,7 +658,7 @@ class _Engine:
             self.ids_alt = torch.empty_like(self.ids)
             ws = int(self.lib.jt_cell_sort_workspace_bytes(self.n, self.grid.bits))
             self.ws = torch.empty(ws, dtype=torch.uint8, device=pos.device)
-            self._sort(first=True)
+            self._sort(first=True, comp_zero=comp_zero)
         self.p = tracker.make_params(self.pos, dt, n_steps, sched_dev, status, self.comp)
         # per-particle path length (indexed by particle, so the sort leaves it be)
         self.path = None
@@ -682,22 +684,22 @@ class _Engine:
                     if chunk > 0:
                         self.stage = _StageFields(f, entries, uid, pos.device, n_steps, chunk, overlap=overlap)
 
-    def _sort(self, first=False):
+    def _sort(self, first=False, comp_zero=False):
+        # Kahan terms that are still zero need no moving
+        moved = None if comp_zero else self.comp
         src_pos = self.out if first else self.pos
         dst_pos = self.pos if first else self.pos_alt
         src_ids = None if first else self.ids
         dst_ids = self.ids if first else self.ids_alt
-        comp_dst = None
-        if self.comp is not None:
-            comp_dst = self.comp_alt
-        L.check(self.lib.jt_cell_sort(C.byref(self.grid), self.n, L.ptr(src_pos), L.ptr(self.comp), L.ptr(src_ids),
+        comp_dst = self.comp_alt if moved is not None else None
+        L.check(self.lib.jt_cell_sort(C.byref(self.grid), self.n, L.ptr(src_pos), L.ptr(moved), L.ptr(src_ids),
                                       L.ptr(dst_pos), L.ptr(comp_dst), L.ptr(dst_ids), L.ptr(self.ws),
                                       self.ws.numel(), self.stream))
-        self.kernels += 5      # keys, two scan levels, scan add, scatter
+        self.kernels += 6      # keys, two scan levels, scan add, slots, gather
         if not first:
             self.pos, self.pos_alt = self.pos_alt, self.pos
             self.ids, self.ids_alt = self.ids_alt, self.ids
-        if self.comp is not None:
+        if moved is not None:
             self.comp, self.comp_alt = self.comp_alt, self.comp
 
     def _stop(self, s, e, staged):
