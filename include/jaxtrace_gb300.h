@@ -522,6 +522,9 @@ int jt_adjoint_rk4(const jt_field* field, const jt_boundary* bc, const jt_adjoin
  * with x fastest (density passes: an x-run of cells is one particle range). */
 #define JT_ORDER_MORTON 0
 #define JT_ORDER_LINEAR 1
+#define JT_ORDER_MORTON_Z 2 /* Morton with z in the lowest bit: 32 cells in a row
+                               are 2 x 4 x 4, four in z, the axis grid nodes
+                               are consecutive in                             */
 typedef struct {
     float origin[3];
     float inv_cell[3];

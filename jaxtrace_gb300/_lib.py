@@ -114,7 +114,7 @@ class AdjointParams(C.Structure):
                 ("work", vp), ("work_bytes", i64), ("stage", vp)]
 
 
-JT_ORDER_MORTON, JT_ORDER_LINEAR = 0, 1
+JT_ORDER_MORTON, JT_ORDER_LINEAR, JT_ORDER_MORTON_Z = 0, 1, 2
 JT_SPH_CUBIC, JT_SPH_WENDLAND, JT_SPH_GAUSSIAN = 0, 1, 2
 
 

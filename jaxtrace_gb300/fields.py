@@ -282,8 +282,9 @@ class _DeviceField:
         return single_blend(self.times, t, **self._blend_args())
 
     def sort_grid(self, bits: int = 7):
-        """Morton cell grid (2^bits per axis over the field's bounding box)
-        used to reorder particles for gather locality.
+        """Morton cell grid (2^bits per axis over the field's bounding box, z
+        in the lowest bit as in the grids' memory) used to reorder particles
+        for gather locality.
 
         The mesh and scattered-node fields keep the bounds of the positions
         they uploaded: reducing 274,625 node positions again for every run
@@ -296,6 +297,7 @@ class _DeviceField:
         g.origin[:] = [float(v) for v in lo]
         g.inv_cell[:] = [float((1 << bits) / e) if e > 0 else 0.0 for e in ext]
         g.bits = bits
+        g.order = L.JT_ORDER_MORTON_Z
         return g
 
     def get_time_bounds(self) -> Tuple[float, float]:
