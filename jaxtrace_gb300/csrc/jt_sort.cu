@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_keys(jt_sort_grid g, const floa
     }
     // z lowest: the 32 cells of a warp are 2 x 4 x 4, four nodes in a row of the
     // grid's memory, half the cache lines of 4 x 4 x 2 (inlet runs of 100 steps:
-    // 2M float32 12.0 -> 11.2 ms, 16.8M bfloat16 34.9 -> 33.0)
+    // 2M float32 12.1 -> 11.5 ms, 16.8M bfloat16 35.4 -> 33.6)
     const uint32_t key = g.order == JT_ORDER_LINEAR ? (((c[2] << g.bits) | c[1]) << g.bits) | c[0]
                          : g.order == JT_ORDER_MORTON_Z ? morton3(c[2], c[1], c[0])
                                                         : morton3(c[0], c[1], c[2]);

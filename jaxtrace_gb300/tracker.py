@@ -49,7 +49,7 @@ class TrackerOptions:
     device_memory_gb   device budget of one trajectory slab
     time_chunk         steps per kernel launch (None: as many as fit)
     sort_every         re-sort particles by cell every k steps for gather
-                       locality (None: on regular grids 50 from 2^18 particles
+                       locality (None: on regular grids 100 from 2^18 particles
                        up, on meshes and scattered nodes 32 from 2^17 up; 0:
                        never)
     sort_bits          cells per axis of that sort, as a power of two
@@ -354,10 +354,10 @@ class ParticleTracker:
         return p
 
     def _sort_every(self, n: int) -> int:
-        """Locality re-sort interval: 50 steps on a regular grid from 2^18
-        particles up (inlet run at 128^3: float32, 2M particles x 400 steps 42.0
-        ms at 50, 42.2 at 34, 42.4 at 100, 43.9 at 200; bfloat16, 16.8M x 200 68.3
-        at 50, 69.2 at 34, 68.7 at 100, 70.9 at 200); 32 on tetrahedral meshes and
+        """Locality re-sort interval: 100 steps on a regular grid from 2^18
+        particles up (16.8M-particle precision workload, 1000 steps: bfloat16 299
+        ms at 50, 290 at 100, 289 at 150, 290 at 200, 297 at 300; float32 412, 407,
+        411, 417 and 431); 32 on tetrahedral meshes and
         scattered nodes, whose lookups lose locality sooner, from 2^17 up (64
         steps, octree, 1M particles: 12.9 ms at 8, 12.5 at 16, 12.3 at 32, 12.4 at
         64, 18.1 unsorted; 200,000 particles 4.2 ms at 32 and 4.7 unsorted, 60,000
@@ -370,7 +370,7 @@ class ParticleTracker:
                 return 0
             if scattered:
                 return 32
-            return 50
+            return 100
         return max(int(se), 0)
 
     def _sort_bits(self) -> int:
