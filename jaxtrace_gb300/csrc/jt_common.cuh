@@ -127,6 +127,14 @@ __device__ __forceinline__ void ldg256(const void* p, uint32_t (&w)[8]) {
         : "l"(p));
 }
 
+// One 256-bit store of a whole 32-byte record: two 128-bit ones each write half
+// of every sector (blending offset quads at 128^3: 5.1 -> 6.2 TB/s).
+__device__ __forceinline__ void stg256(void* p, const uint4& a, const uint4& b) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+                 "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
+
 template <>
 __device__ __forceinline__ PairVal load_pair<JT_STORE_F32>(const void* base, int64_t rec) {
     uint32_t w[8];

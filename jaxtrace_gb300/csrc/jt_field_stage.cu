@@ -71,9 +71,9 @@ __global__ void __launch_bounds__(kBlock) k_stage_f32q(jt_grid_field F, const jt
         for (int c = 0; c < 4; ++c)
             v[c] = blend_cv<EXACT, JT_STORE_F32>(pv[c], e, splat(e.wa), splat(e.wb), e.form == JT_BLEND_WEIGHTED);
         char* slot = out + (int64_t)jj * S * 48;
-        float4* a = reinterpret_cast<float4*>(slot + node * 32);
-        a[0] = make_float4(v[0].xy.x, v[0].xy.y, v[1].xy.x, v[1].xy.y);
-        a[1] = make_float4(v[2].xy.x, v[2].xy.y, v[3].xy.x, v[3].xy.y);
+        const auto u = [](float f) { return __float_as_uint(f); };
+        stg256(slot + node * 32, make_uint4(u(v[0].xy.x), u(v[0].xy.y), u(v[1].xy.x), u(v[1].xy.y)),
+               make_uint4(u(v[2].xy.x), u(v[2].xy.y), u(v[3].xy.x), u(v[3].xy.y)));
         reinterpret_cast<float4*>(slot + S * 32)[node] = make_float4(v[0].z, v[1].z, v[2].z, v[3].z);
     }
 }
@@ -156,9 +156,7 @@ __global__ void __launch_bounds__(kStageBlock16, 16) k_stage_f16(jt_grid_field F
                          V3{c10.xy.x, c10.xy.y, c10.z}, V3{c11.xy.x, c11.xy.y, c11.z}};
         uint4 a, b;
         encode_quad(u, a, b);
-        uint4* o = out + 2 * ((int64_t)j * N + node);
-        o[0] = a;
-        o[1] = b;
+        stg256(out + 2 * ((int64_t)j * N + node), a, b);
     }
 }
 
@@ -252,9 +250,7 @@ __global__ void __launch_bounds__(kStageBlock16, 16) k_stage_tile(jt_grid_field 
         }
         uint4 a, b;
         encode_quad(u, a, b);
-        uint4* o = out + 2 * ((int64_t)jj * N + node);
-        o[0] = a;
-        o[1] = b;
+        stg256(out + 2 * ((int64_t)jj * N + node), a, b);
     }
 }
 
