@@ -663,6 +663,7 @@ class TimeSeriesField(_DeviceField):
         q.points = block.data_ptr()
         self._dev["points"] = block
         L.check(lib.jt_nearest_lists_fill(C.byref(q), start.data_ptr(), L.stream_ptr()))
+        torch.cuda.current_stream().synchronize()     # the field may be used on any stream next
         q.storage |= L.JT_NEAREST_LISTS
 
     def _device_pairs(self):
@@ -964,6 +965,7 @@ class FEMTimeSeriesField(TimeSeriesField):
                                           L.stream_ptr()))
             d["sub_start"], d["sub_elems"] = start, elems
             f.sub_start, f.sub_elems = start.data_ptr(), elems.data_ptr()
+        torch.cuda.current_stream().synchronize()     # the field may be used on any stream next
 
     def __repr__(self) -> str:
         return (f"FEMTimeSeriesField(data={self.data.shape}, times={self.times.shape}, "
