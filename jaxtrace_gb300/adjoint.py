@@ -149,6 +149,20 @@ class AdjointRK4:
                 "stride": stride}
 
 
+def _quads_pay(n: int, n_steps: int, nodes: int) -> bool:
+    """Whether the backward blends its fields as quads (48 B a node, a quarter of
+    the kernel's loads) instead of node records (16 B).  Quads need a particle
+    per node: with fewer the wider records are mostly read for one particle,
+    and writing them costs more than the loads they save.  And they need steps
+    enough to earn the look at the free memory and the larger buffer (25 us).
+    Backward pass of 20 steps, node records against quads: 96^3 nodes, 100,000
+    particles 1.90 and 2.48 ms, 300,000 2.59 and 3.16, 1M 5.18 and 4.99; 64^3,
+    20,000 1.00 and 1.06, 100,000 1.19 and 1.33, 300,000 1.99 and 1.96, 1M 4.46
+    and 4.08; 32^3, 100,000 1.06 and 1.06, 300,000 1.81 and 1.73; 17^3, 20,000
+    0.80 and 0.82, 300,000 1.76 and 1.75, 1M 4.15 and 4.05."""
+    return n >= nodes and n * n_steps >= 1 << 22
+
+
 def _make_function():
     import torch
 
@@ -241,9 +255,9 @@ def _make_function():
             if solver.stage_fields:
                 # 3 schedule entries (stage times) per step, and room for one segment's fields
                 src = ctx.sched.view(-1, 4, 8)[:, :3].contiguous().view(-1, 8)
-                # as quads where there is room: a quarter of the kernel's loads
                 quad_floats = 3 * min(k, ctx.n_steps) * (solver.nodes + (solver.nodes & 1)) * 12
-                quads = quad_floats * 4 <= torch.cuda.mem_get_info(lam.device)[0] // 4
+                quads = _quads_pay(n, ctx.n_steps, solver.nodes) and \
+                    quad_floats * 4 <= torch.cuda.mem_get_info(lam.device)[0] // 4
                 a.stage_storage = L.JT_STORE_STAGE_F32Q if quads else L.JT_STORE_STAGE_F32
                 stage = torch.empty(quad_floats if quads else 3 * k * solver.nodes * 4, dtype=torch.float32,
                                     device=lam.device)
