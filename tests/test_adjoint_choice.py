@@ -7,6 +7,7 @@ import pytest
 
 import jaxtrace_gb300 as jt
 from jaxtrace_gb300 import adjoint as A
+from jaxtrace_gb300 import tracker as T
 from jaxtrace_gb300 import workloads as W
 
 F32 = np.float32
@@ -18,6 +19,20 @@ F32 = np.float32
                                                  (20_000, 20, 17 ** 3, False), (1_000_000, 20, 96 ** 3, True)])
 def test_rule(n, steps, nodes, quads):
     assert A._quads_pay(n, steps, nodes) == quads
+
+
+def test_small_forward_passes_are_turned_away_before_any_work(monkeypatch):
+    g = np.linspace(0, 1, 33).astype(F32)
+    s = A.AdjointRK4(np.linspace(0, 1, 4).astype(F32), g, g, g, "clamp")
+
+    def looked(*a):
+        raise AssertionError("the entries were looked at")
+    monkeypatch.setattr(T, "_stage_entries", looked)
+    assert s._blend_ahead(None, 20, np.zeros((20_000, 3), F32)) is None
+    assert s._blend_ahead(None, 0, np.zeros((20_000, 3), F32)) is None
+    with pytest.raises(AssertionError):
+        monkeypatch.setattr(A, "_torch", lambda: None)
+        s._blend_ahead(None, 50, np.zeros((1_000_000, 3), F32))
 
 
 @pytest.mark.gpu
