@@ -113,11 +113,11 @@ class TrackerOptions:
     autotune: bool = False
     cuda_graph: bool = False
     stage_fields: bool = True
-    stage_min_gain: float = 1.0
     stage_chunk: int = 32
     stage_overlap: bool = True
     row_sink: Optional[Callable[[int, np.ndarray, Optional[np.ndarray], np.ndarray], None]] = None
     record_path_length: bool = False
+    stage_min_gain: float = 1.0     # last, so that the options before it keep their positions
 
     def estimate_batch_size(self, n_particles: int, n_timesteps: int) -> int:
         """tracker.py:142-153."""
