@@ -1,0 +1,52 @@
+"""Single SPH terms, where no sum of many hides their rounding."""
+import numpy as np
+import pytest
+
+from jaxtrace_gb300.density import SPHDensityEstimator
+
+pytestmark = pytest.mark.gpu
+F32 = np.float32
+
+
+def _one_term(kind, lo, hi):
+    """(q, term of one particle at q smoothing lengths as a share of the term at
+    0) for queries that have that particle alone in their support, among many
+    more in the same rows of cells."""
+    import torch
+    rng = np.random.default_rng(3)
+    h = 0.02
+    g = 0.5 + 0.143 * np.arange(-3, 4)
+    q0 = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3).astype(F32)
+    d = rng.normal(size=q0.shape)
+    d *= (rng.uniform(lo, hi, len(q0)) * h / np.linalg.norm(d, axis=1))[:, None]
+    near = (q0 + d).astype(F32)
+    fill = rng.random((400_000, 3)).astype(F32)
+    cell = 0.5 + 0.143 * np.rint((fill.astype(np.float64) - 0.5) / 0.143).clip(-3, 3)
+    fill = fill[np.linalg.norm(fill - cell, axis=1) > (2.1 + hi) * h]     # outside the partner's support too
+    P = np.concatenate([near, fill])
+    s = SPHDensityEstimator(P, dimensions="3d", smoothing_length=h, kernel_type=kind, normalize=False)
+    at = s._density_sum(torch.from_numpy(np.concatenate([q0, near])).cuda()).cpu().numpy()
+    r = np.linalg.norm(near.astype(np.float64) - q0, axis=1) / np.float64(F32(h))
+    return r, at[:len(q0)] / at[len(q0):]
+
+
+@pytest.mark.parametrize("kind", ["cubic_spline", "wendland"])
+def test_near_terms_round_once(kind):
+    """Below q = 0.05 the kernel's float32 value is its last rounding, half a unit
+    in the last place of [0.5, 1), and the rounding of q, which moves it by at
+    most 10 q^2 (8 2^-24): 2^-25 and 1.2e-8.  Wendland's adds two products'
+    and the slope's roundings of 1 - q: five more of 2^-24 and 20 q 2^-25."""
+    r, got = _one_term(kind, 0.001, 0.05)
+    if kind == "cubic_spline":
+        want, tol = 1 - 1.5 * r ** 2 + 0.75 * r ** 3, 2.0 ** -25 + 1.2e-8
+    else:
+        want, tol = (1 - r) ** 4 * (1 + 4 * r), 6 * 2.0 ** -24
+    assert np.abs(got - want).max() <= tol
+
+
+def test_both_branches_of_the_spline():
+    """Across q = 1: value 0.25 with slope -0.75; the rounding of q (8 2^-24) and
+    four roundings of values up to 1 stay below 12 2^-24."""
+    r, got = _one_term("cubic_spline", 0.9, 1.1)
+    want = np.where(r <= 1, 1 - 1.5 * r ** 2 + 0.75 * r ** 3, 0.25 * (2 - r) ** 3)
+    assert np.abs(got - want).max() <= 12 * 2.0 ** -24
