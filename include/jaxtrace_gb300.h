@@ -601,9 +601,8 @@ typedef struct {
                                   particles (N,4) {x,y,z,mass} in one 16-byte
                                   record; 2: particle pairs (ceil(N/2),8)
                                   {x0,x1,y0,y1,z0,z1,mass0,mass1} (16-byte
-                                  aligned; an odd N pads the last pair), for
-                                  finite masses.  1 and 2 leave masses unused
-                                  and need h NULL                             */
+                                  aligned; an odd N pads the last pair).  1
+                                  and 2 leave masses unused and need h NULL   */
     const float* particles;    /* device (N,3) or (N,4) in cell order        */
     const float* masses;       /* device (N) in cell order, or NULL (unit masses) */
     const float* h;            /* device (N) in cell order, or NULL (h_const) */

@@ -194,110 +194,117 @@ __global__ void __launch_bounds__(kBlock) k_sph(jt_sph_params P) {
         const float r2lim = fminf(r2max, sup >= 1.8e19f ? r2max : sup * sup);
         // the cutoff beyond the support, and h^2 well inside float32's range
         const float tiny = 1e-14f * hh * hh;
-        const bool whole = r2max >= sup * sup && tiny > 1e-34f && hh < 1e15f;
+        bool cut = !COUNT && KERN != JT_SPH_GAUSSIAN && P.packed == 2 && r2max >= sup * sup && tiny > 1e-34f && hh < 1e15f;
         // rows of the cell box whose slab lies beyond the support sphere are
         // skipped and the rest trimmed in x (with a margin: only whole
         // cells that cannot hold a term are dropped)
         const float csy = 1.0f / g.inv_cell[1], csz = DIM == 3 ? 1.0f / g.inv_cell[2] : 0.0f;
-        for (int z = z0; z <= z1; ++z) {
-            const float dzr = DIM == 3 ? fmaxf(fmaxf(g.origin[2] + z * csz - qz, qz - (g.origin[2] + (z + 1) * csz)),
-                                               0.0f)
-                                       : 0.0f;
-            for (int y = y0; y <= y1; ++y) {
-                const float dyr = fmaxf(fmaxf(g.origin[1] + y * csy - qy, qy - (g.origin[1] + (y + 1) * csy)), 0.0f);
-                const float rem = r2lim - dyr * dyr - dzr * dzr;
-                if (rem < -1e-6f * r2lim) continue;
-                const float rx = sqrtf(fmaxf(rem, 0.0f)) * 1.0001f + 1e-7f;
-                const int xa = max(x0, cell_of(qx - rx, g.origin[0], g.inv_cell[0], lim));
-                const int xb = min(x1, cell_of(qx + rx, g.origin[0], g.inv_cell[0], lim));
-                if (xa > xb) continue;
-                uint32_t b, e;
-                row_range(P.cell_end, xa, xb, y, z, g.bits, b, e);
-                float part = 0.0f;
-                if (P.packed == 2) {
-                    // pairs of particles (x0 x1 y0 y1 z0 z1 m0 m1): two
-                    // candidates per iteration in float32x2 arithmetic, their
-                    // terms added in particle order as one at a time
-                    if (COUNT) n_cand += e - b;
-                    const float2 nqx = make_float2(-qx, -qx), nqy = make_float2(-qy, -qy),
-                                 nqz = make_float2(-qz, -qz), inv2 = make_float2(inv, inv);
-                    uint32_t j = b;
-                    if (j < e && (j & 1u)) {  // a row that starts on a pair's second particle
-                        part = sph_pair_one<DIM, KERN, COUNT>(P.particles, j, qx, qy, qz, inv, r2lim, part, n_in);
-                        ++j;
-                    }
-                    const float4* p4 = reinterpret_cast<const float4*>(P.particles);
-                    if (!COUNT && KERN != JT_SPH_GAUSSIAN && whole) {
-                        // no support test and no choice between the spline's two
-                        // branches: 4M positions piled at two walls, h = 0.02,
-                        // 18.0 -> 15.9 ms a pass; L1 79 %, issue 66 %, FMA 65 %, 21.6
-                        // of 32 lanes active (rows of different lengths).  Loops
-                        // unrolled 1 or 4 times and 6 or 8 blocks/SM: no faster
-                        float2 sum = make_float2(0.0f, 0.0f);
+        // Without a support test every candidate's mass is multiplied, by 0 beyond
+        // the support.  A mass that is not finite gives NaN there, so a query
+        // whose sum is not finite is summed again with the test.
+        for (;; cut = false) {
+            acc = 0.0;
+            for (int z = z0; z <= z1; ++z) {
+                const float dzr = DIM == 3 ? fmaxf(fmaxf(g.origin[2] + z * csz - qz, qz - (g.origin[2] + (z + 1) * csz)),
+                                                   0.0f)
+                                           : 0.0f;
+                for (int y = y0; y <= y1; ++y) {
+                    const float dyr = fmaxf(fmaxf(g.origin[1] + y * csy - qy, qy - (g.origin[1] + (y + 1) * csy)), 0.0f);
+                    const float rem = r2lim - dyr * dyr - dzr * dzr;
+                    if (rem < -1e-6f * r2lim) continue;
+                    const float rx = sqrtf(fmaxf(rem, 0.0f)) * 1.0001f + 1e-7f;
+                    const int xa = max(x0, cell_of(qx - rx, g.origin[0], g.inv_cell[0], lim));
+                    const int xb = min(x1, cell_of(qx + rx, g.origin[0], g.inv_cell[0], lim));
+                    if (xa > xb) continue;
+                    uint32_t b, e;
+                    row_range(P.cell_end, xa, xb, y, z, g.bits, b, e);
+                    float part = 0.0f;
+                    if (P.packed == 2) {
+                        // pairs of particles (x0 x1 y0 y1 z0 z1 m0 m1): two
+                        // candidates per iteration in float32x2 arithmetic, their
+                        // terms added in particle order as one at a time
+                        if (COUNT) n_cand += e - b;
+                        const float2 nqx = make_float2(-qx, -qx), nqy = make_float2(-qy, -qy),
+                                     nqz = make_float2(-qz, -qz), inv2 = make_float2(inv, inv);
+                        uint32_t j = b;
+                        if (j < e && (j & 1u)) {  // a row that starts on a pair's second particle
+                            part = sph_pair_one<DIM, KERN, COUNT>(P.particles, j, qx, qy, qz, inv, r2lim, part, n_in);
+                            ++j;
+                        }
+                        const float4* p4 = reinterpret_cast<const float4*>(P.particles);
+                        if (cut) {
+                            // no support test and no choice between the spline's two
+                            // branches: 4M positions piled at two walls, h = 0.02,
+                            // 18.0 -> 15.9 ms a pass; L1 79 %, issue 66 %, FMA 65 %, 21.6
+                            // of 32 lanes active (rows of different lengths).  Loops
+                            // unrolled 1 or 4 times and 6 or 8 blocks/SM: no faster
+                            float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll 2
+                            for (; j + 1 < e; j += 2) {
+                                const float4 u = __ldg(p4 + j), w = __ldg(p4 + j + 1);
+                                const float2 dx = __fadd2_rn(make_float2(u.x, u.y), nqx);
+                                const float2 dy = __fadd2_rn(make_float2(u.z, u.w), nqy);
+                                float2 d2 = make_float2(tiny, tiny);
+                                if (DIM == 3) {
+                                    const float2 dz = __fadd2_rn(make_float2(w.x, w.y), nqz);
+                                    d2 = __ffma2_rn(dz, dz, d2);
+                                }
+                                d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, d2));
+                                sum = __ffma2_rn(make_float2(w.z, w.w), sph_cut2<KERN>(d2, inv), sum);
+                            }
+                            part += kSphCut<KERN> * (sum.x + sum.y);
+                        }
 #pragma unroll 2
                         for (; j + 1 < e; j += 2) {
-                            const float4 u = __ldg(p4 + j), w = __ldg(p4 + j + 1);
+                            const float4 u = __ldg(p4 + j), w = __ldg(p4 + j + 1);  // j even: pair j/2
                             const float2 dx = __fadd2_rn(make_float2(u.x, u.y), nqx);
                             const float2 dy = __fadd2_rn(make_float2(u.z, u.w), nqy);
-                            float2 d2 = make_float2(tiny, tiny);
-                            if (DIM == 3) {
-                                const float2 dz = __fadd2_rn(make_float2(w.x, w.y), nqz);
-                                d2 = __ffma2_rn(dz, dz, d2);
+                            const float2 dz = DIM == 3 ? __fadd2_rn(make_float2(w.x, w.y), nqz) : make_float2(0.0f, 0.0f);
+                            const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                            const float2 sh =
+                                sph_shape2<KERN>(__fmul2_rn(make_float2(fast_dist(d2.x), fast_dist(d2.y)), inv2));
+                            if (d2.x <= r2lim) {
+                                part = fmaf(w.z, sh.x, part);
+                                if (COUNT) ++n_in;
                             }
-                            d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, d2));
-                            sum = __ffma2_rn(make_float2(w.z, w.w), sph_cut2<KERN>(d2, inv), sum);
+                            if (d2.y <= r2lim) {
+                                part = fmaf(w.w, sh.y, part);
+                                if (COUNT) ++n_in;
+                            }
                         }
-                        part += kSphCut<KERN> * (sum.x + sum.y);
-                    }
-#pragma unroll 2
-                    for (; j + 1 < e; j += 2) {
-                        const float4 u = __ldg(p4 + j), w = __ldg(p4 + j + 1);  // j even: pair j/2
-                        const float2 dx = __fadd2_rn(make_float2(u.x, u.y), nqx);
-                        const float2 dy = __fadd2_rn(make_float2(u.z, u.w), nqy);
-                        const float2 dz = DIM == 3 ? __fadd2_rn(make_float2(w.x, w.y), nqz) : make_float2(0.0f, 0.0f);
-                        const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-                        const float2 sh =
-                            sph_shape2<KERN>(__fmul2_rn(make_float2(fast_dist(d2.x), fast_dist(d2.y)), inv2));
-                        if (d2.x <= r2lim) {
-                            part = fmaf(w.z, sh.x, part);
-                            if (COUNT) ++n_in;
-                        }
-                        if (d2.y <= r2lim) {
-                            part = fmaf(w.w, sh.y, part);
-                            if (COUNT) ++n_in;
-                        }
-                    }
-                    if (j < e)  // a row that ends on a pair's first particle
-                        part = sph_pair_one<DIM, KERN, COUNT>(P.particles, j, qx, qy, qz, inv, r2lim, part, n_in);
-                } else if (P.packed) {
-                    // {x, y, z, m} records; FMA-contracted distance (no parity
-                    // constraint on the density passes)
-                    const float4* p4 = reinterpret_cast<const float4*>(P.particles);
-                    if (COUNT) n_cand += e - b;
+                        if (j < e)  // a row that ends on a pair's first particle
+                            part = sph_pair_one<DIM, KERN, COUNT>(P.particles, j, qx, qy, qz, inv, r2lim, part, n_in);
+                    } else if (P.packed) {
+                        // {x, y, z, m} records; FMA-contracted distance (no parity
+                        // constraint on the density passes)
+                        const float4* p4 = reinterpret_cast<const float4*>(P.particles);
+                        if (COUNT) n_cand += e - b;
 #pragma unroll 4
-                    for (uint32_t j = b; j < e; ++j) {
-                        const float4 r = __ldg(p4 + j);
-                        const float dx = r.x - qx, dy = r.y - qy, dz = DIM == 3 ? r.z - qz : 0.0f;
-                        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        if (d2 <= r2lim) {
-                            part = fmaf(r.w, sph_shape<KERN>(fast_dist(d2) * inv), part);
-                            if (COUNT) ++n_in;
+                        for (uint32_t j = b; j < e; ++j) {
+                            const float4 r = __ldg(p4 + j);
+                            const float dx = r.x - qx, dy = r.y - qy, dz = DIM == 3 ? r.z - qz : 0.0f;
+                            const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                            if (d2 <= r2lim) {
+                                part = fmaf(r.w, sph_shape<KERN>(fast_dist(d2) * inv), part);
+                                if (COUNT) ++n_in;
+                            }
+                        }
+                    } else {
+                        for (uint32_t j = b; j < e; ++j) {
+                            const float dx = __ldg(P.particles + 3 * (int64_t)j) - qx;
+                            const float dy = __ldg(P.particles + 3 * (int64_t)j + 1) - qy;
+                            const float dz = DIM == 3 ? __ldg(P.particles + 3 * (int64_t)j + 2) - qz : 0.0f;
+                            const float d2 = dx * dx + dy * dy + dz * dz;
+                            if (d2 <= r2lim) {
+                                const float m = P.masses != nullptr ? __ldg(P.masses + j) : 1.0f;
+                                part += m * sph_shape<KERN>(fast_dist(d2) * inv);
+                            }
                         }
                     }
-                } else {
-                    for (uint32_t j = b; j < e; ++j) {
-                        const float dx = __ldg(P.particles + 3 * (int64_t)j) - qx;
-                        const float dy = __ldg(P.particles + 3 * (int64_t)j + 1) - qy;
-                        const float dz = DIM == 3 ? __ldg(P.particles + 3 * (int64_t)j + 2) - qz : 0.0f;
-                        const float d2 = dx * dx + dy * dy + dz * dz;
-                        if (d2 <= r2lim) {
-                            const float m = P.masses != nullptr ? __ldg(P.masses + j) : 1.0f;
-                            part += m * sph_shape<KERN>(fast_dist(d2) * inv);
-                        }
-                    }
+                    acc += (double)part * (double)sigma;
                 }
-                acc += (double)part * (double)sigma;
             }
+            if (!cut || isfinite(acc)) break;
         }
     } else {
         for (int z = z0; z <= z1; ++z) {

@@ -529,13 +529,7 @@ class SPHDensityEstimator:
         p.grid = cl.grid
         p.reach[:] = cl.reach(search)
         p.masses = None
-        if h_sorted is None and m_sorted is not None and not bool(torch.isfinite(m_sorted).all()):
-            # the paired loop multiplies every candidate's mass, by 0 beyond the
-            # support: masses that are not finite need the one that tests it
-            P4 = torch.cat([cl.sorted, m_sorted[:, None]], dim=1).contiguous()
-            p.packed = 1
-            p.particles = P4.data_ptr()
-        elif h_sorted is None:
+        if h_sorted is None:
             # uniform h: two 16-byte loads per two candidates
             P4 = pair_records(cl.sorted, m_sorted)
             p.packed = 2

@@ -50,3 +50,33 @@ def test_both_branches_of_the_spline():
     r, got = _one_term("cubic_spline", 0.9, 1.1)
     want = np.where(r <= 1, 1 - 1.5 * r ** 2 + 0.75 * r ** 3, 0.25 * (2 - r) ** 3)
     assert np.abs(got - want).max() <= 12 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("kind,reach", [("cubic_spline", 2.0), ("wendland", 1.0)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_masses_that_are_not_finite_in_pair_records(monkeypatch, kind, reach, bad):
+    """Pair records take any mass, and a finite check costs no call a look at all
+    masses: the sums that the particle reaches are not finite, the others are
+    those without it, though their rows of cells hold it too (to 1e-5: the
+    order of a cell's particles differs from run to run)."""
+    import torch
+    from jaxtrace_gb300 import density
+    rng = np.random.default_rng(1)
+    h = 0.05
+    P = torch.from_numpy(rng.random((100_000, 3)).astype(F32)).cuda()
+    q = P[:20_000].contiguous()
+    m = rng.uniform(0.5, 2.0, len(P)).astype(F32)
+    paired = []
+    monkeypatch.setattr(density, "pair_records", lambda *a, f=density.pair_records: paired.append(1) or f(*a))
+    sums = []
+    for k in (None, 7, 8):                       # either half of a pair, by the cells' order
+        if k is not None:
+            m[k] = bad
+        s = SPHDensityEstimator(P, dimensions="3d", smoothing_length=h, kernel_type=kind, masses=m, normalize=False)
+        sums.append(s._density_sum(q).cpu().numpy())
+    assert len(paired) == 3
+    d = np.stack([np.linalg.norm((q - P[k]).double().cpu().numpy(), axis=1) for k in (7, 8)]) / np.float64(F32(h))
+    for rho, near in zip(sums[1:], (d[0], d.min(axis=0))):
+        inside, outside = near < reach - 1e-5, near > reach + 1e-5
+        assert inside.any() and not np.isfinite(rho[inside]).any()
+        assert np.allclose(rho[outside], sums[0][outside], rtol=1e-5)
