@@ -14,6 +14,8 @@
 // block never visits; their terms are below exp(-radius^2/2h^2).
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "jt_internal.h"
 #include "jt_kernels.cuh"
 
@@ -170,7 +172,8 @@ __device__ __forceinline__ float sph_pair_one(const float* pairs, uint32_t j, fl
 
 // COUNT: also count the candidate pairs examined and those inside the
 // support (P.counters), a separate instance so the plain one keeps its loop.
-template <int DIM, int KERN, bool COUNT = false>
+// CUT: pair records without a support test, where rows are long enough for it.
+template <int DIM, int KERN, bool COUNT = false, bool CUT = false>
 __global__ void __launch_bounds__(kBlock) k_sph(jt_sph_params P) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n_queries) return;
@@ -194,7 +197,7 @@ __global__ void __launch_bounds__(kBlock) k_sph(jt_sph_params P) {
         const float r2lim = fminf(r2max, sup >= 1.8e19f ? r2max : sup * sup);
         // the cutoff beyond the support, and h^2 well inside float32's range
         const float tiny = 1e-14f * hh * hh;
-        bool cut = !COUNT && KERN != JT_SPH_GAUSSIAN && P.packed == 2 && r2max >= sup * sup && tiny > 1e-34f && hh < 1e15f;
+        bool cut = CUT && r2max >= sup * sup && tiny > 1e-34f && hh < 1e15f;
         // rows of the cell box whose slab lies beyond the support sphere are
         // skipped and the rest trimmed in x (with a margin: only whole
         // cells that cannot hold a term are dropped)
@@ -221,8 +224,7 @@ __global__ void __launch_bounds__(kBlock) k_sph(jt_sph_params P) {
                     float part = 0.0f;
                     if (P.packed == 2) {
                         // pairs of particles (x0 x1 y0 y1 z0 z1 m0 m1): two
-                        // candidates per iteration in float32x2 arithmetic, their
-                        // terms added in particle order as one at a time
+                        // candidates per iteration in float32x2 arithmetic
                         if (COUNT) n_cand += e - b;
                         const float2 nqx = make_float2(-qx, -qx), nqy = make_float2(-qy, -qy),
                                      nqz = make_float2(-qz, -qz), inv2 = make_float2(inv, inv);
@@ -233,11 +235,11 @@ __global__ void __launch_bounds__(kBlock) k_sph(jt_sph_params P) {
                         }
                         const float4* p4 = reinterpret_cast<const float4*>(P.particles);
                         if (cut) {
-                            // no support test and no choice between the spline's two
-                            // branches: 4M positions piled at two walls, h = 0.02,
-                            // 18.0 -> 15.9 ms a pass; L1 79 %, issue 66 %, FMA 65 %, 21.6
-                            // of 32 lanes active (rows of different lengths).  Loops
-                            // unrolled 1 or 4 times and 6 or 8 blocks/SM: no faster
+                            // no support test, and one sum a lane, joined at the
+                            // row's end: 4M positions piled at two walls, h = 0.02,
+                            // 18.0 -> 16.3 ms a pass; 21.6 of 32 lanes active (rows of
+                            // different lengths).  Loops unrolled 1 or 4 times and 6
+                            // or 8 blocks/SM: no faster
                             float2 sum = make_float2(0.0f, 0.0f);
 #pragma unroll 2
                             for (; j + 1 < e; j += 2) {
@@ -254,6 +256,7 @@ __global__ void __launch_bounds__(kBlock) k_sph(jt_sph_params P) {
                             }
                             part += kSphCut<KERN> * (sum.x + sum.y);
                         }
+                        // with the test: terms added in particle order, as one at a time
 #pragma unroll 2
                         for (; j + 1 < e; j += 2) {
                             const float4 u = __ldg(p4 + j), w = __ldg(p4 + j + 1);  // j even: pair j/2
@@ -697,6 +700,27 @@ __global__ void __launch_bounds__(kBlock) k_kde_points(jt_kde_params P, const fl
 
 using namespace jt;
 
+// Whether rows hold candidates enough, on average over the grid, for the loop
+// without a support test: its sums are joined once a row and its parameters
+// take registers, and a term costs less.  Kernel with the test against
+// without, uniform positions: rows of 0.5 (3-D, 20,000 positions, h = 0.02)
+// 47.4 and 49.0 us; 1.1 (1M, Wendland, h = 0.005) 78.3 and 87.0; 3.9 (1M,
+// h = 0.014) 727 and 713; 4.4 (4M, Wendland, h = 0.005) 417 and 427; 6.8 (4M,
+// h = 0.005) 1050 and 1024, (Wendland, h = 0.01) 951 and 941; 21 (4M, h = 0.02)
+// 9616 and 8918; 2-D, 20,000: 4.4 11.3 and 11.5, 7.5 16.6 and 16.5.
+constexpr double kSphCutRow = 6.0;
+
+static bool sph_cut(const jt_sph_params& p) {
+    if (p.packed != 2 || p.h != nullptr || p.kernel == JT_SPH_GAUSSIAN) return false;
+    double row = p.n_particles;
+    const double cells = (double)(1 << p.grid.bits);
+    for (int a = 0; a < p.dims; ++a)
+        if (p.grid.inv_cell[a] > 0.0f) row /= cells;
+    const double reach = std::min((double)p.radius, (p.kernel == JT_SPH_CUBIC ? 2.0 : 1.0) * p.h_const);
+    if (p.grid.inv_cell[0] > 0.0f) row *= std::min(2.0 * reach * p.grid.inv_cell[0] + 1.0, cells);
+    return row >= kSphCutRow;
+}
+
 extern "C" int jt_sph_density(const jt_sph_params* p, void* stream) {
     if (p == nullptr) return set_error(JT_ERR_INVALID, "params is NULL");
     if (p->dims != 2 && p->dims != 3) return set_error(JT_ERR_INVALID, "dims must be 2 or 3");
@@ -720,6 +744,13 @@ extern "C" int jt_sph_density(const jt_sph_params* p, void* stream) {
         else if (p->dims == 3 && p->kernel == JT_SPH_WENDLAND) k_sph<3, JT_SPH_WENDLAND, true><<<gb, kBlock, 0, st>>>(*p);
         else if (p->dims == 3) k_sph<3, JT_SPH_GAUSSIAN, true><<<gb, kBlock, 0, st>>>(*p);
         else return set_error(JT_ERR_UNSUPPORTED, "SPH counters are for 3-D");
+        return cuda_status(cudaGetLastError(), "SPH kernel launch");
+    }
+    if (sph_cut(*p)) {
+        if (p->dims == 3 && p->kernel == JT_SPH_CUBIC) k_sph<3, JT_SPH_CUBIC, false, true><<<gb, kBlock, 0, st>>>(*p);
+        else if (p->dims == 3) k_sph<3, JT_SPH_WENDLAND, false, true><<<gb, kBlock, 0, st>>>(*p);
+        else if (p->kernel == JT_SPH_CUBIC) k_sph<2, JT_SPH_CUBIC, false, true><<<gb, kBlock, 0, st>>>(*p);
+        else k_sph<2, JT_SPH_WENDLAND, false, true><<<gb, kBlock, 0, st>>>(*p);
         return cuda_status(cudaGetLastError(), "SPH kernel launch");
     }
 #define JT_SPH_LAUNCH(D, K) k_sph<D, K><<<gb, kBlock, 0, st>>>(*p)

@@ -80,3 +80,42 @@ def test_masses_that_are_not_finite_in_pair_records(monkeypatch, kind, reach, ba
         inside, outside = near < reach - 1e-5, near > reach + 1e-5
         assert inside.any() and not np.isfinite(rho[inside]).any()
         assert np.allclose(rho[outside], sums[0][outside], rtol=1e-5)
+
+
+@pytest.mark.parametrize("kind", ["cubic_spline", "wendland"])
+@pytest.mark.parametrize("dims", [2, 3])
+def test_rows_choose_the_loop(kind, dims):
+    """Sparse rows keep the tested loop, whose sums are those of its terms in
+    particle order, bit for bit; long ones take the other.  Cells are set
+    here, so that one row holds them all or hardly any."""
+    import ctypes as C
+
+    import torch
+    from jaxtrace_gb300 import _lib as L
+    from jaxtrace_gb300 import density as D
+    rng = np.random.default_rng(4)
+    n, h = 6000, (0.05 if dims == 3 else 0.01)
+    P = rng.random((n, 3)).astype(F32)
+    if dims == 2:
+        P[:, 2] = 0
+    dev = torch.from_numpy(P).cuda()
+    got = {}
+    for cell in (1.0, 0.01):
+        cl = D.CellList(dev, [0.0] * 3, [1.0, 1.0, 1.0 if dims == 3 else 0.0], cell, dims)
+        out = {}
+        for packed in (1, 2):
+            m = torch.ones(n, device="cuda")
+            rec = D.pair_records(cl.sorted, m) if packed == 2 else torch.cat([cl.sorted, m[:, None]], 1).contiguous()
+            o = torch.empty(n, dtype=torch.float64, device="cuda")
+            p = L.SphParams()
+            p.dims, p.kernel = dims, D._SPH_KERNELS[kind]
+            p.n_particles = p.n_queries = n
+            p.radius, p.h_const, p.grid, p.packed = 3 * h, h, cl.grid, packed
+            p.reach[:] = cl.reach(2 * h)
+            p.particles, p.cell_end, p.queries, p.out = (t.data_ptr() for t in (rec, cl.cell_end, cl.sorted, o))
+            L.check(L.load().jt_sph_density(C.byref(p), L.stream_ptr()))
+            out[packed] = o.cpu().numpy()
+        got[cell] = out
+        assert np.allclose(out[1], out[2], rtol=1e-5)
+    assert np.array_equal(got[0.01][1], got[0.01][2])          # one or two candidates a row: the same loop's terms
+    assert not np.array_equal(got[1.0][1], got[1.0][2])        # thousands a row: the other
