@@ -435,13 +435,13 @@ constexpr int kKbT = 8;  // the 3-D KDE's grid tile edge
 // adjacent rows, one wavefront a load.  The tile stays 8^3 so that the dilated
 // box of particles each tile visits stays small.
 //
-// Sums run in float32 over at most kKdFlush / 8 = 128 particles a thread, then
-// over the eight groups in pairs, then in float64: an eighth of the float64
-// additions that every thread's own sums would take, which at two lanes a cycle
-// and SM were a third of the time.  3,000,017 particles, 100^3 points: 22.0 ms
-// with eight points a thread (64 threads, float64 sums of their own every 240
-// particles, bound by shared memory), 15.5 ms with 32 in the same box, 10 ms with
-// the ball below; the FMA pipe is 73 % busy.
+// Sums run in float32 over at most kKdSpan particles of a thread, all further
+// ones in float64: a sixteenth of the float64 additions that every thread's own
+// sums of 240 particles and 8 points would take, which at two lanes a cycle and
+// SM were a third of the time.  Adding the groups in float32 first would save
+// no time.  3,000,017 particles, 100^3 points: 21.4 ms with eight points a thread
+// (64 threads, bound by shared memory), 12.5 ms with 32 and the ball below (11.8
+// with 240 particles in a sum, and larger errors).
 //
 // The particles summed are those of the cells that meet the ball of kKdReach
 // radii around the tile: 6 bandwidths for the default radius of 5.  A box of one
@@ -454,11 +454,11 @@ constexpr int kKbT = 8;  // the 3-D KDE's grid tile edge
 constexpr int kKdThreads = 128;
 constexpr int kKdGroups = kKdThreads / 16;
 constexpr int kKdChunk = 256;   // particles in shared memory: 3 x 256 x 32 B = 24 KB
-constexpr int kKdFlush = 1024;  // particles between float64 sums
+constexpr int kKdSpan = 128;    // particles in a float32 sum, at most
 constexpr float kKdReach = 1.2f;
 constexpr int kKdRows = 4 * kKdThreads;  // rows of cells listed at a time
 static_assert(kKdGroups * kKbT * kKbT * kKbT <= 3 * kKdChunk * kKbT, "the groups' sums fit the factors' memory");
-static_assert(kKdFlush % kKdChunk == 0, "sums after whole chunks");
+static_assert(kKdChunk / kKdGroups <= kKdSpan, "a chunk fits a sum");
 
 __global__ void __launch_bounds__(kKdThreads, 5) k_kde_grid3_blocked(jt_kde_params P) {
     __shared__ __align__(16) float fac[3][kKdChunk][kKbT];
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kKdThreads, 5) k_kde_grid3_blocked(jt_kde_para
     float2 q[2][4][2];
 #pragma unroll
     for (int i = 0; i < 16; ++i) q[i >> 3][(i >> 1) & 3][i & 1] = make_float2(0.0f, 0.0f);
-    // the groups' float32 sums into float64: thread t owns points 4t .. 4t + 3
+    // every group's float32 sums into float64: thread t owns points 4t .. 4t + 3
     const auto flush = [&]() {
         float* red = &fac[0][0][0];
         __syncthreads();
@@ -516,22 +516,18 @@ __global__ void __launch_bounds__(kKdThreads, 5) k_kde_grid3_blocked(jt_kde_para
                 q[i][j][0] = q[i][j][1] = make_float2(0.0f, 0.0f);
             }
         __syncthreads();
-        float4 v[kKdGroups];
 #pragma unroll
-        for (int k = 0; k < kKdGroups; ++k) v[k] = *reinterpret_cast<const float4*>(red + k * 512 + 4 * t);
-#pragma unroll
-        for (int w = kKdGroups / 2; w > 0; w >>= 1)
-#pragma unroll
-            for (int k = 0; k < w; ++k)
-                v[k] = make_float4(v[k].x + v[k + w].x, v[k].y + v[k + w].y, v[k].z + v[k + w].z, v[k].w + v[k + w].w);
-        acc[0] += (double)v[0].x;
-        acc[1] += (double)v[0].y;
-        acc[2] += (double)v[0].z;
-        acc[3] += (double)v[0].w;
+        for (int k = 0; k < kKdGroups; ++k) {
+            const float4 v = *reinterpret_cast<const float4*>(red + k * 512 + 4 * t);
+            acc[0] += (double)v.x;
+            acc[1] += (double)v.y;
+            acc[2] += (double)v.z;
+            acc[3] += (double)v.w;
+        }
         __syncthreads();
     };
     unsigned long long visits = 0;
-    int summed = 0;  // particles since the last flush
+    int summed = 0;  // particles a thread may have summed since the last flush
     const int ny = hi1 - lo1 + 1, rows = ny * (hi2 - lo2 + 1);
     for (int r0 = 0; r0 < rows; r0 += kKdRows) {
         // the rows' particle ranges, four rows a thread, and where each ends
@@ -640,8 +636,8 @@ __global__ void __launch_bounds__(kKdThreads, 5) k_kde_grid3_blocked(jt_kde_para
                     q[i][3][1] = __ffma2_rn(splat(p23.y), z23, q[i][3][1]);
                 }
             }
-            summed += held;
-            if (summed >= kKdFlush) {
+            summed += (held + kKdGroups - 1) / kKdGroups;
+            if (summed + kKdChunk / kKdGroups > kKdSpan) {
                 flush();
                 summed = 0;
             } else {
