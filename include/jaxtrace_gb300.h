@@ -628,7 +628,9 @@ typedef struct {
     int32_t n_particles;
     int32_t res[3];            /* grid points per axis (x, y, z; z = 1 in 2-D) */
     float half_inv_h2;         /* 0.5 / h^2                                   */
-    float radius;              /* particles farther than this along an axis from every grid point of a tile are skipped */
+    float radius;              /* particles within this along each axis of a grid point of a tile are summed, farther
+                                  ones may be skipped: on 3-D grids also those up to 1.1 radii away are summed where
+                                  radius is 5 bandwidths or more; cells are taken whole */
     jt_sort_grid grid;         /* cell grid of the particle cell list         */
     const float* axis[3];      /* device float32 grid coordinates per axis    */
     const float* particles;    /* device (N,3) in cell order                  */

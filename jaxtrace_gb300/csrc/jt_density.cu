@@ -10,8 +10,9 @@
 // KDE grid: exp(-|g-p|^2/2h^2) = ex * ey * ez factorises per axis, so a block
 // owning an 8x8x8 tile of grid points computes 24 exponentials per particle
 // (8 per axis) instead of 512 and forms the products from shared memory.
-// Particles more than `radius` from the tile along an axis lie in cells the
-// block never visits; their terms are below exp(-radius^2/2h^2).
+// Cells that lie more than `radius` from the tile along an axis are left out
+// (on 3-D grids only where they lie outside the ball below too); their terms
+// are below exp(-radius^2/2h^2).
 #include <stdint.h>
 
 #include <algorithm>
@@ -436,26 +437,26 @@ constexpr int kKbT = 8;  // the 3-D KDE's grid tile edge
 // box of particles each tile visits stays small.
 //
 // Sums run in float32 over at most kKdSpan particles of a thread, all further
-// ones in float64: a sixteenth of the float64 additions that every thread's own
-// sums of 240 particles and 8 points would take, which at two lanes a cycle and
-// SM were a third of the time.  Adding the groups in float32 first would save
-// no time.  3,000,017 particles, 100^3 points: 21.4 ms with eight points a thread
-// (64 threads, bound by shared memory), 12.5 ms with 32 and the ball below (11.8
-// with 240 particles in a sum, and larger errors).
+// ones in float64, by way of shared memory (32 float64 sums of a thread's own
+// would take 64 registers).  3,000,017 particles, 100^3 points: 21.4 ms with eight
+// points a thread (64 threads, bound by shared memory), 13.0 ms with 32 and the
+// cells below; with 240 particles in a sum 5 % less time and larger errors.
 //
-// The particles summed are those of the cells that meet the ball of kKdReach
-// radii around the tile: 6 bandwidths for the default radius of 5.  A box of one
-// radius (plus its cells' remainders, up to half a radius) has 1.5 times the
-// volume and drops more: a Gaussian's mass beyond 5 sigma on an axis is 6e-7,
-// beyond a distance of 6 sigma 7e-8.  The estimator cuts its cells to suit.  The
-// rows of cells are listed first, a row a thread and step, and their particles
-// then dealt out in whole chunks: walking the rows one by one cost as much as
-// the finer cells saved.
+// The particles summed are those of the cells that meet the tile grown by one
+// radius along each axis, and, where a radius is 5 bandwidths or more (the
+// default), also those within kKdReach radii of the tile: with the finer cells
+// that the estimator then cuts, of which less lies beyond the radius, that keeps
+// the error below that of cells of half a radius: 3,000,017 particles, 100^3
+// points, median 5.9e-8 against 7.0e-8.  The grown tile alone would take 4 % less
+// time with 8.8e-8, a rim of 1.2 radii 8 % more with 5.2e-8.  The rows of cells
+// are listed first, a row a thread and step, and their particles then dealt out
+// in whole chunks: walking the rows one by one cost as much as the finer cells
+// saved.
 constexpr int kKdThreads = 128;
 constexpr int kKdGroups = kKdThreads / 16;
 constexpr int kKdChunk = 256;   // particles in shared memory: 3 x 256 x 32 B = 24 KB
 constexpr int kKdSpan = 128;    // particles in a float32 sum, at most
-constexpr float kKdReach = 1.2f;
+constexpr float kKdReach = 1.1f, kKdReachFrom = 4.999f;
 constexpr int kKdRows = 4 * kKdThreads;  // rows of cells listed at a time
 static_assert(kKdGroups * kKbT * kKbT * kKbT <= 3 * kKdChunk * kKbT, "the groups' sums fit the factors' memory");
 static_assert(kKdChunk / kKdGroups <= kKdSpan, "a chunk fits a sum");
@@ -483,13 +484,20 @@ __global__ void __launch_bounds__(kKdThreads, 5) k_kde_grid3_blocked(jt_kde_para
     const int lim = (1 << g.bits) - 1;
     const float x_lo = gcoord[0][0], x_hi = gcoord[0][n0 - 1], y_lo = gcoord[1][0], y_hi = gcoord[1][n1 - 1];
     const float z_lo = gcoord[2][0], z_hi = gcoord[2][n2 - 1];
-    const float reach = kKdReach * P.radius, far2 = reach * reach;
+    const bool wide = P.radius * sqrtf(2.0f * P.half_inv_h2) >= kKdReachFrom;
+    const float reach = wide ? kKdReach * P.radius : P.radius, far2 = reach * reach;
     const int lo0 = cell_of(x_lo - reach, g.origin[0], g.inv_cell[0], lim);
     const int hi0 = cell_of(x_hi + reach, g.origin[0], g.inv_cell[0], lim);
     const int lo1 = cell_of(y_lo - reach, g.origin[1], g.inv_cell[1], lim);
     const int hi1 = cell_of(y_hi + reach, g.origin[1], g.inv_cell[1], lim);
     const int lo2 = cell_of(z_lo - reach, g.origin[2], g.inv_cell[2], lim);
     const int hi2 = cell_of(z_hi + reach, g.origin[2], g.inv_cell[2], lim);
+    const int bx0 = cell_of(x_lo - P.radius, g.origin[0], g.inv_cell[0], lim);
+    const int bx1 = cell_of(x_hi + P.radius, g.origin[0], g.inv_cell[0], lim);
+    const int by0 = cell_of(y_lo - P.radius, g.origin[1], g.inv_cell[1], lim);
+    const int by1 = cell_of(y_hi + P.radius, g.origin[1], g.inv_cell[1], lim);
+    const int bz0 = cell_of(z_lo - P.radius, g.origin[2], g.inv_cell[2], lim);
+    const int bz1 = cell_of(z_hi + P.radius, g.origin[2], g.inv_cell[2], lim);
     // gap between the tile and cells c of an axis, less 1e-3 of a cell for the
     // rounding of the particles' cells; the end cells reach to infinity
     const auto gap = [lim](int c, float org, float inv, float lo, float hi) {
@@ -541,14 +549,20 @@ __global__ void __launch_bounds__(kKdThreads, 5) k_kde_grid3_blocked(jt_kde_para
                 const float gz = gap(cz, g.origin[2], g.inv_cell[2], z_lo, z_hi);
                 const float gy = gap(cy, g.origin[1], g.inv_cell[1], y_lo, y_hi);
                 const float rem = far2 - gy * gy - gz * gz;
+                // the row's cells of the box and of the ball: one run, as both hold the tile's
+                int xa = lim + 1, xb = -1;
+                if (cy >= by0 && cy <= by1 && cz >= bz0 && cz <= bz1) {
+                    xa = bx0;
+                    xb = bx1;
+                }
                 if (rem >= 0.0f) {
                     const float w = sqrtf(rem) * 1.0001f;
-                    const int xa = max(lo0, cell_of(x_lo - w, g.origin[0], g.inv_cell[0], lim));
-                    const int xb = min(hi0, cell_of(x_hi + w, g.origin[0], g.inv_cell[0], lim));
-                    uint32_t e = 0;
-                    if (xa <= xb) row_range(P.cell_end, xa, xb, cy, cz, g.bits, first[k], e);
-                    cnt[k] = e > first[k] ? e - first[k] : 0u;
+                    xa = min(xa, max(lo0, cell_of(x_lo - w, g.origin[0], g.inv_cell[0], lim)));
+                    xb = max(xb, min(hi0, cell_of(x_hi + w, g.origin[0], g.inv_cell[0], lim)));
                 }
+                uint32_t e = 0;
+                if (xa <= xb) row_range(P.cell_end, xa, xb, cy, cz, g.bits, first[k], e);
+                cnt[k] = e > first[k] ? e - first[k] : 0u;
             }
             mine += cnt[k];
         }

@@ -6,8 +6,9 @@ Semantics (exact, not truncated):
 * KDE: ``mean_j (2 pi)^{-d/2} exp(-|q - p_j|^2 / 2h^2)``, the formula of the
   JAX and pure-NumPy paths (kde.py:249-282), with Scott/Silverman bandwidths
   (kernels.py:30-68) and the grid normalisation of kde.py:205-240 done in
-  float64.  Terms farther than ``cutoff_sigmas * h`` along an axis are
-  skipped (each is below exp(-cutoff_sigmas^2/2); 5 sigma by default).
+  float64.  Every term within ``cutoff_sigmas * h`` along each axis is
+  summed; farther ones may be left out (each is below
+  exp(-cutoff_sigmas^2/2); 5 sigma by default).
   SciPy's ``gaussian_kde(bw_method=h)`` (the reference's fallback when SciPy
   is present, kde.py:273-275) scales the kernel by the data covariance and is
   a different estimator; it is not reproduced.
@@ -247,10 +248,12 @@ class KDEEstimator:
         ax = [torch.from_numpy(np.ascontiguousarray(a, dtype=F32)).cuda() for a in axes]
         lo = [min(float(pts[:, a].min()), float(axes[a][0])) for a in range(dims)] + [0.0] * (3 - dims)
         hi = [max(float(pts[:, a].max()), float(axes[a][-1])) for a in range(dims)] + [0.0] * (3 - dims)
-        # the 3-D grid kernel cuts a ball out of the cells: about 32 particles
-        # per cell, between a twelfth and half of the radius, hug it
+        # from 5 sigma the 3-D grid kernel takes a rim of cells beyond the
+        # cutoff by itself (jt_kde_grid): about 32 particles per cell, between a
+        # twelfth and half of the radius, hug it.  Below that the cells of half
+        # a radius are the rim: what they hold beyond a short cutoff counts
         cell = None
-        if dims == 3:
+        if dims == 3 and self.cutoff_sigmas >= 5.0:
             radius = float(self.cutoff_sigmas * self.h)
             vol = float(np.prod([max(b - a, 1e-30) for a, b in zip(lo, hi)]))
             cell = max(min((32.0 * vol / max(int(pts.shape[0]), 1)) ** (1.0 / 3.0), radius / 2.0), radius / 12.0, 1e-6)
