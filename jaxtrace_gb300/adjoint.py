@@ -128,6 +128,7 @@ class AdjointRK4:
         A run whose particles would not pay for the usual two fields a step is
         turned away before any entry is looked at: that took 40 to 70 us of the
         host, 5 % of a small gradient's forward pass."""
+        from .fields import room_for
         from .tracker import _stage_entries, _stage_gain
         if n_steps < 1 or x0.shape[0] < 1 or \
                 _stage_gain(x0.shape[0], n_steps, L.JT_RK4, (2 * n_steps - 1,), self.nodes) < 1.0:
@@ -139,7 +140,7 @@ class AdjointRK4:
         lo, hi = uid[3 * begin], uid[3 * np.minimum(begin + self.k, n_steps) - 1] + 1
         slots = int((hi - lo).max())
         if _stage_gain(x0.shape[0], n_steps, L.JT_RK4, uid, self.nodes) < 1.0 or \
-                slots * stride * 48 > torch.cuda.mem_get_info(x0.device)[0] // 4:
+                not room_for(slots * stride * 48, x0.device):
             return None
         every = host.reshape(n_steps, 4)[:, :3].reshape(-1)
         first = np.ones(len(every), dtype=bool)
@@ -170,6 +171,8 @@ def _quads_pay(n: int, n_steps: int, nodes: int) -> bool:
 
 def _make_function():
     import torch
+
+    from .fields import room_for
 
     class AdjointFunction(torch.autograd.Function):
         @staticmethod
@@ -261,8 +264,7 @@ def _make_function():
                 # 3 schedule entries (stage times) per step, and room for one segment's fields
                 src = ctx.sched.view(-1, 4, 8)[:, :3].contiguous().view(-1, 8)
                 quad_floats = 3 * min(k, ctx.n_steps) * (solver.nodes + (solver.nodes & 1)) * 12
-                quads = _quads_pay(n, ctx.n_steps, solver.nodes) and \
-                    quad_floats * 4 <= torch.cuda.mem_get_info(lam.device)[0] // 4
+                quads = _quads_pay(n, ctx.n_steps, solver.nodes) and room_for(quad_floats * 4, lam.device)
                 a.stage_storage = L.JT_STORE_STAGE_F32Q if quads else L.JT_STORE_STAGE_F32
                 stage = torch.empty(quad_floats if quads else 3 * k * solver.nodes * 4, dtype=torch.float32,
                                     device=lam.device)

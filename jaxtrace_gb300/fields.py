@@ -35,6 +35,18 @@ def _torch_cuda():
     return torch
 
 
+def room_for(nbytes: int, device=None) -> bool:
+    """Whether an optional buffer of that size takes at most a quarter of the
+    device memory to be had: what the driver has free and, asked for only where
+    that is too little, what torch's allocator keeps without using (the blocks
+    of an earlier call, which the same call would otherwise see as taken)."""
+    import torch
+    free = torch.cuda.mem_get_info(device)[0]
+    if nbytes <= free // 4:
+        return True
+    return nbytes <= (free + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)) // 4
+
+
 def _mark_near_degenerate(tet_box, tet_geom) -> int:
     """Flag the near-degenerate tetrahedra of a field's device box records
     (jt_mark_near_degenerate); returns how many there are."""
@@ -655,7 +667,7 @@ class TimeSeriesField(_DeviceField):
         total = C.c_int64(0)
         L.check(lib.jt_nearest_lists_count(C.byref(q), start.data_ptr(), C.byref(total), L.stream_ptr()))
         size = int(lib.jt_nearest_lists_bytes(C.byref(q), total.value))
-        if size > torch.cuda.mem_get_info()[0] // 4:
+        if not room_for(size):
             return
         block = torch.empty(size, dtype=torch.uint8, device="cuda")
         pts = self._dev["points"]
