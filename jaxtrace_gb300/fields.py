@@ -953,10 +953,11 @@ class FEMTimeSeriesField(TimeSeriesField):
     def _upload_filters(self, f, d):
         """The geometry records with the filter records behind them
         (jt_fem_filters_build), and the sub-cell lists without the entries
-        those rule out (jt_fem_prune_fill); the mesh keeps its own lists."""
+        those rule out (jt_fem_prune_fill); the mesh keeps its own lists.
+        Either is left out where it does not fit: the field needs neither."""
         torch = _torch_cuda()
         M = f.n_tets
-        if not 0 < M <= 1 << 26:
+        if not 0 < M <= 1 << 26 or not room_for(M * 96):
             return
         block = torch.empty((M * 24,), dtype=torch.float32, device="cuda")
         block[:M * 16] = d["tet_geom"].reshape(-1)
@@ -965,18 +966,19 @@ class FEMTimeSeriesField(TimeSeriesField):
         lib = L.load()
         L.check(lib.jt_fem_filters_build(C.byref(f), L.stream_ptr()))
         f.sub_div |= L.JT_FEM_FILTERS
-        if self.fem_mesh.sub_div:
+        if self.fem_mesh.sub_div and room_for(2 * d["sub_start"].numel() * 4):
             h = self.fem_mesh
             eps = np.nextafter(h._eps(h.sub_div, h.cell_size64).astype(F32), F32(np.inf))
             start = torch.empty_like(d["sub_start"])
             total = C.c_int64(0)
             L.check(lib.jt_fem_prune_count(C.byref(f), eps.ctypes.data, start.data_ptr(), C.byref(total),
                                            L.stream_ptr()))
-            elems = torch.empty(max(total.value, 1), dtype=torch.int32, device="cuda")
-            L.check(lib.jt_fem_prune_fill(C.byref(f), eps.ctypes.data, start.data_ptr(), elems.data_ptr(),
-                                          L.stream_ptr()))
-            d["sub_start"], d["sub_elems"] = start, elems
-            f.sub_start, f.sub_elems = start.data_ptr(), elems.data_ptr()
+            if room_for(total.value * 4):
+                elems = torch.empty(max(total.value, 1), dtype=torch.int32, device="cuda")
+                L.check(lib.jt_fem_prune_fill(C.byref(f), eps.ctypes.data, start.data_ptr(), elems.data_ptr(),
+                                              L.stream_ptr()))
+                d["sub_start"], d["sub_elems"] = start, elems
+                f.sub_start, f.sub_elems = start.data_ptr(), elems.data_ptr()
         torch.cuda.current_stream().synchronize()     # the field may be used on any stream next
 
     def __repr__(self) -> str:
@@ -1197,7 +1199,8 @@ class OctreeFEMTimeSeriesFieldOptimized(_DeviceField):
     def _upload_descent(self, f, d, bfs):
         """The breadth-first tree, and behind it the locator block
         (jt_mesh_locator_build) of as many levels as the tree has, at most
-        JT_MESH_LOCATOR_MAX_DEPTH: a table of 2^21 cells, 16 MB, at 7."""
+        JT_MESH_LOCATOR_MAX_DEPTH: a table of 2^21 cells, 16 MB, at 7, and 96 B a
+        tetrahedron.  The tree alone where that does not fit."""
         torch = _torch_cuda()
         m, lib = self.octree_mesh, L.load()
         desc, dtab = bfs
@@ -1205,6 +1208,8 @@ class OctreeFEMTimeSeriesFieldOptimized(_DeviceField):
         listed = int(m.info.n_elem_entries) == f.n_tets
         S = locator_splits(m.nodes_min[0], m.nodes_max[0], depth) if depth > 0 and listed else None
         size = int(lib.jt_mesh_locator_bytes(len(dtab), f.n_tets, depth)) if S is not None else dtab.nbytes
+        if S is not None and not room_for(size):
+            S, size = None, dtab.nbytes
         block = torch.empty(size, dtype=torch.uint8, device="cuda")
         block[:dtab.nbytes] = torch.from_numpy(dtab.view(np.uint8).reshape(-1)).cuda()
         d["desc"], d["dtab"] = torch.from_numpy(desc).cuda(), block
