@@ -26,6 +26,7 @@ JT_TILE, JT_TILE_NODES = 4, 125
 JT_GRID_CLAMP, JT_GRID_ZERO, JT_GRID_NAN, JT_GRID_PERIODIC = 0, 1, 2, 3
 JT_BLEND_WEIGHTED, JT_BLEND_LERP_FWD, JT_BLEND_LERP_BWD, JT_BLEND_SAME_A, JT_BLEND_SAME_B = 0, 1, 2, 3, 4
 JT_EULER, JT_RK2, JT_RK4 = 0, 1, 2
+EVALS = {JT_EULER: 1, JT_RK2: 2, JT_RK4: 4}     # evaluations of the field in a step
 JT_BC_NONE, JT_BC_PERIODIC, JT_BC_REFLECTIVE, JT_BC_CLAMP, JT_BC_ABSORBING = 0, 1, 2, 3, 4
 JT_INLET_OFF, JT_INLET_GRID = 0, 1
 JT_ARITH_EXACT, JT_ARITH_COMPENSATED = 0, 1

@@ -17,6 +17,7 @@ bracketing snapshots).  Calling ``sample_at_positions`` runs a CUDA kernel;
 from __future__ import annotations
 
 import ctypes as C
+import threading
 import warnings
 from typing import Optional, Tuple
 
@@ -54,6 +55,12 @@ def _mark_near_degenerate(tet_box, tet_geom) -> int:
     L.check(L.load().jt_mark_near_degenerate(tet_box.data_ptr(), tet_geom.data_ptr(), tet_box.shape[0],
                                              C.byref(n), L.stream_ptr()))
     return int(n.value)
+
+
+def _copy_struct(s):
+    out = type(s)()
+    C.memmove(C.byref(out), C.byref(s), C.sizeof(s))
+    return out
 
 
 def _as_f32(a) -> np.ndarray:
@@ -251,11 +258,24 @@ def build_tile_snapshots(data: np.ndarray, dims, periodic: bool, storage: int, d
     return res, base, (TX, TY, TZ)
 
 
+_RECORDS_LOCK = threading.Lock()
+
+
 class _DeviceField:
-    """Shared plumbing: snapshot times, blend semantics and the jt_field struct."""
+    """Shared plumbing: snapshot times, blend semantics and the jt_field struct.
+
+    The mesh and scattered-node fields have optional lookup records (octree
+    locator, hash-grid filters, candidate lists): the same bits sooner, for some
+    time and memory.  They are built once the evaluations asked of the field
+    would have saved that time (``_field_for``), so that a probe of a few points
+    pays for none, and no field for more than it has spent without them."""
 
     _semantics = "numpy"
     _uploaded_bounds = None     # (lo, hi) of the node positions on the device
+    _records = True             # built for the present upload, or none to build
+    _records_cost = 0.0         # us to build
+    _records_gain = (0.0, 0.0)  # us saved by an evaluation in a thread's chain, and by any (_field_for)
+    _saved = 0.0                # us that they would have saved so far
 
     def _init_time(self, times, interpolation, extrapolation, storage, semantics):
         self.times = _as_f32(times)
@@ -320,9 +340,36 @@ class _DeviceField:
 
     # -- device sampling --
     def jt_field(self):
-        """The ctypes ``jt_field`` of this field (device buffers built on first use)."""
+        """The ctypes ``jt_field`` of this field (device buffers built on first
+        use, the optional records included)."""
         self._device()
+        self._build_once()
         return self._cfield
+
+    def _field_for(self, n: int, evals: int):
+        """``jt_field`` for ``n`` threads of ``evals`` evaluations each, one after the
+        other: such a launch waits for the chain of one thread and, with many
+        threads, for the sum of all."""
+        self._device()
+        if not self._records:
+            chain, each = self._records_gain
+            self._saved += evals * (chain + n * each)
+            if self._saved >= self._records_cost:
+                self._build_once()
+        return self._cfield
+
+    def _build_once(self):
+        import torch
+        if self._records or torch.cuda.is_current_stream_capturing():
+            return                      # the build reads its sizes back: not while a graph is captured
+        with _RECORDS_LOCK:
+            if self._records:
+                return
+            try:
+                self._build_records()   # new buffers and a new descriptor: launches in flight keep theirs
+            except torch.cuda.OutOfMemoryError:
+                pass
+            self._records = True
 
     def sample_at_positions(self, query_positions, t, *, arith=None):
         """Velocities at (M,3) positions and time t (fields/base.py:106-122).
@@ -348,7 +395,7 @@ class _DeviceField:
         e = self.blend_at(t)
         blend = L.Blend.from_buffer_copy(e.tobytes())
         status = torch.zeros(1, dtype=torch.int32, device="cuda")
-        L.check(L.load().jt_field_sample(C.byref(self._cfield), C.byref(blend),
+        L.check(L.load().jt_field_sample(C.byref(self._field_for(q.shape[0], 1)), C.byref(blend),
                                          self._default_arith() if arith is None else int(arith),
                                          L.ptr(q), L.ptr(out), q.shape[0], L.ptr(status), L.stream_ptr()))
         return out if is_tensor else out.cpu().numpy()
@@ -359,6 +406,13 @@ class _DeviceField:
 
     def evaluate(self, a, b):
         return self(a, b)
+
+    def _uploaded(self, cost, gain):
+        """The upload is done; its optional records cost and save so much."""
+        import torch
+        torch.cuda.current_stream().synchronize()     # the field may be used on any stream next
+        self._records_cost, self._records_gain, self._saved = cost, gain, 0.0
+        self._records = False
 
     def sample_at_time(self, t):
         """All node values at time t (time_series.py:306), blended on the device."""
@@ -650,33 +704,46 @@ class TimeSeriesField(_DeviceField):
         q.point_ids = self._dev["ids"].data_ptr()
         q.cell_start = self._dev["start"].data_ptr()
         q.pairs = pairs.data_ptr()
-        self._upload_lists(q)
         self._cnear = q
         self._cfield = L.Field(kind=L.JT_FIELD_NEAREST, nearest=C.pointer(q))
+        self._uploaded(*self._lists_cost())
 
-    def _upload_lists(self, q):
-        """The candidate lists of the nearest-node search behind the sorted
-        nodes (jt_nearest_lists_fill): about four cells per node and eight
-        16-byte records per cell."""
+    def _lists_cost(self):
+        """Candidate lists against rings of cells, 20 RK4 steps over 274,625 nodes:
+        2000 particles 1.27 and 0.35 ms, 1M 6.9 and 2.2; over 2,197 nodes 0.93 and
+        0.31, 4.5 and 1.2.  Built in 10.3 ms there, 4.9 for 117,649, 0.6 for 2,197."""
+        return 500.0 + 0.037 * self.N, (9.0, 5e-5)
+
+    def _build_records(self):
+        q = self._with_lists(self._cnear)
+        if q is not None:
+            self._cnear, self._cfield = q, L.Field(kind=L.JT_FIELD_NEAREST, nearest=C.pointer(q))
+
+    def _with_lists(self, q):
+        """The descriptor with the candidate lists of the nearest-node search
+        behind the sorted nodes (jt_nearest_lists_fill): about four cells per
+        node and eight 16-byte records per cell.  None without them."""
         torch = _torch_cuda()
         lib = L.load()
         cells = int(lib.jt_nearest_lists_cells(C.byref(q)))
         if cells == 0:
-            return
+            return None
         start = torch.empty(cells + 1, dtype=torch.int32, device="cuda")
         total = C.c_int64(0)
         L.check(lib.jt_nearest_lists_count(C.byref(q), start.data_ptr(), C.byref(total), L.stream_ptr()))
         size = int(lib.jt_nearest_lists_bytes(C.byref(q), total.value))
         if not room_for(size):
-            return
+            return None
         block = torch.empty(size, dtype=torch.uint8, device="cuda")
         pts = self._dev["points"]
         block[:pts.numel() * 4] = pts.view(torch.uint8).reshape(-1)
+        q = _copy_struct(q)
         q.points = block.data_ptr()
-        self._dev["points"] = block
         L.check(lib.jt_nearest_lists_fill(C.byref(q), start.data_ptr(), L.stream_ptr()))
         torch.cuda.current_stream().synchronize()     # the field may be used on any stream next
         q.storage |= L.JT_NEAREST_LISTS
+        self._dev["lists"] = block
+        return q
 
     def _device_pairs(self):
         self._device()
@@ -946,11 +1013,23 @@ class FEMTimeSeriesField(TimeSeriesField):
         f.sub_div = h.sub_div
         f.sub_start, f.sub_elems = d["sub_start"].data_ptr(), d["sub_elems"].data_ptr()
         f.near_degenerate = int(self.n_near_degenerate > 0)
-        self._upload_filters(f, d)
         self._cfem = f
         self._cfield = L.Field(kind=L.JT_FIELD_FEM, fem=C.pointer(f))
+        # filters, pruned lists and candidate lists against plain scans and rings, 20
+        # RK4 steps on 1,572,864 tetrahedra: 2000 particles 1.35 and 0.60 ms, 1M 13.7
+        # and 5.2; on 10,368 tetrahedra 1.21 and 0.57, 7.8 and 3.7.  Built, candidate
+        # lists included, in 30.8 ms there, 11.9 for 663,552, 1.1 for 10,368
+        self._uploaded(self._lists_cost()[0] + 400.0 + 0.0125 * f.n_tets, (10.0, 1e-4))
 
-    def _upload_filters(self, f, d):
+    def _build_records(self):
+        f = _copy_struct(self._cfem)
+        q = self._with_lists(self._cnear)
+        if q is not None:
+            self._cnear = f.nearest = q
+        self._add_filters(f, self._dev)
+        self._cfem, self._cfield = f, L.Field(kind=L.JT_FIELD_FEM, fem=C.pointer(f))
+
+    def _add_filters(self, f, d):
         """The geometry records with the filter records behind them
         (jt_fem_filters_build), and the sub-cell lists without the entries
         those rule out (jt_fem_prune_fill); the mesh keeps its own lists.
@@ -961,7 +1040,7 @@ class FEMTimeSeriesField(TimeSeriesField):
             return
         block = torch.empty((M * 24,), dtype=torch.float32, device="cuda")
         block[:M * 16] = d["tet_geom"].reshape(-1)
-        d["tet_geom"] = block
+        d["filters"] = block
         f.tet_geom = block.data_ptr()
         lib = L.load()
         L.check(lib.jt_fem_filters_build(C.byref(f), L.stream_ptr()))
@@ -977,7 +1056,7 @@ class FEMTimeSeriesField(TimeSeriesField):
                 elems = torch.empty(max(total.value, 1), dtype=torch.int32, device="cuda")
                 L.check(lib.jt_fem_prune_fill(C.byref(f), eps.ctypes.data, start.data_ptr(), elems.data_ptr(),
                                               L.stream_ptr()))
-                d["sub_start"], d["sub_elems"] = start, elems
+                d["pruned_start"], d["pruned_elems"] = start, elems
                 f.sub_start, f.sub_elems = start.data_ptr(), elems.data_ptr()
         torch.cuda.current_stream().synchronize()     # the field may be used on any stream next
 
@@ -1192,34 +1271,41 @@ class OctreeFEMTimeSeriesFieldOptimized(_DeviceField):
         f.near_degenerate = int(self.n_near_degenerate > 0)
         bfs = breadth_first_descent(m.nodes)
         if bfs is not None:
-            self._upload_descent(f, d, bfs)
+            d["desc"], d["dtab"] = (torch.from_numpy(a).cuda() for a in bfs)
+            f.desc, f.dtab = d["desc"].data_ptr(), d["dtab"].data_ptr()
         self._cmesh = f
         self._cfield = L.Field(kind=L.JT_FIELD_MESH, mesh=C.pointer(f))
+        # locator and filters against the descent and plain scans, 20 RK4 steps on
+        # 1,572,864 tetrahedra: 2000 particles 0.68 and 0.55 ms, 1M 5.4 and 3.9; on
+        # 663,552 1.40 and 0.78, 9.9 and 5.7.  Built in 3.2 ms there, 0.9 for
+        # 663,552, 0.3 for 10,368
+        self._uploaded(250.0 + 0.002 * f.n_tets, (5.0, 2e-5))
 
-    def _upload_descent(self, f, d, bfs):
-        """The breadth-first tree, and behind it the locator block
+    def _build_records(self):
+        """The breadth-first tree with the locator block behind it
         (jt_mesh_locator_build) of as many levels as the tree has, at most
         JT_MESH_LOCATOR_MAX_DEPTH: a table of 2^21 cells, 16 MB, at 7, and 96 B a
         tetrahedron.  The tree alone where that does not fit."""
         torch = _torch_cuda()
-        m, lib = self.octree_mesh, L.load()
-        desc, dtab = bfs
+        m, lib, d, f = self.octree_mesh, L.load(), self._dev, _copy_struct(self._cmesh)
         depth = min(int(m.info.max_tree_depth), m.max_depth, L.JT_MESH_LOCATOR_MAX_DEPTH)
-        listed = int(m.info.n_elem_entries) == f.n_tets
-        S = locator_splits(m.nodes_min[0], m.nodes_max[0], depth) if depth > 0 and listed else None
-        size = int(lib.jt_mesh_locator_bytes(len(dtab), f.n_tets, depth)) if S is not None else dtab.nbytes
-        if S is not None and not room_for(size):
-            S, size = None, dtab.nbytes
+        if "dtab" not in d or depth < 1 or int(m.info.n_elem_entries) != f.n_tets:
+            return
+        S = locator_splits(m.nodes_min[0], m.nodes_max[0], depth)
+        size = int(lib.jt_mesh_locator_bytes(f.n_nodes, f.n_tets, depth))
+        if S is None or not room_for(size):
+            return
         block = torch.empty(size, dtype=torch.uint8, device="cuda")
-        block[:dtab.nbytes] = torch.from_numpy(dtab.view(np.uint8).reshape(-1)).cuda()
-        d["desc"], d["dtab"] = torch.from_numpy(desc).cuda(), block
-        f.desc, f.dtab = d["desc"].data_ptr(), block.data_ptr()
-        if S is not None:
-            where = C.c_int32(0)
-            splits = torch.from_numpy(S).cuda()
-            L.check(lib.jt_mesh_locator_build(C.byref(f), depth, splits.data_ptr(), C.byref(where),
-                                              L.stream_ptr()))
+        dtab = d["dtab"].view(torch.uint8).reshape(-1)
+        block[:dtab.numel()] = dtab
+        f.dtab = block.data_ptr()
+        where = C.c_int32(0)
+        splits = torch.from_numpy(S).cuda()
+        L.check(lib.jt_mesh_locator_build(C.byref(f), depth, splits.data_ptr(), C.byref(where), L.stream_ptr()))
+        if where.value:
             f.locator = where.value
+            d["locator"] = block
+            self._cmesh, self._cfield = f, L.Field(kind=L.JT_FIELD_MESH, mesh=C.pointer(f))
 
     def _device_pairs(self):
         self._device()

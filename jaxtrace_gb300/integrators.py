@@ -72,7 +72,7 @@ def _step(code: int, x, t, dt, field_fn):
     arr = (L.Blend * 3).from_buffer_copy(blends.tobytes())
     out = torch.empty_like(xin)
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
-    L.check(L.load().jt_integrator_step(C.byref(field.jt_field()), arr, code, field._default_arith(),
+    L.check(L.load().jt_integrator_step(C.byref(field._field_for(n, L.EVALS[code])), arr, code, field._default_arith(),
                                         float(F32(dt_arr.mean()) if dt_arr.ndim else dt_arr), L.ptr(dtpp),
                                         L.ptr(xin), L.ptr(out), n, L.ptr(status), L.stream_ptr()))
     return out if is_tensor else out.cpu().numpy()

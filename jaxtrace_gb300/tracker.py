@@ -726,7 +726,7 @@ class _Engine:
                 p.schedule = self.stage.sched.data_ptr()
             else:
                 if self.field_c is None:
-                    self.field_c = self.field.jt_field()
+                    self.field_c = self.field._field_for(self.n, self.n_steps * L.EVALS[self.t._code])
                 field_c = self.field_c
                 p.schedule = self.sched.data_ptr()
             p.pos = self.pos.data_ptr()
@@ -841,6 +841,7 @@ class EnsembleBatch:
         """Record one pass in a CUDA graph (after one eager pass that loads
         the library and sets kernel attributes outside the capture)."""
         import torch
+        self.tracker._field.jt_field()      # a pass that is captured is replayed: with every record
         self._pass()
         torch.cuda.synchronize()
         g = torch.cuda.CUDAGraph()
@@ -1017,8 +1018,7 @@ def _stage_gain(n: int, n_steps: int, integrator: int, uid, nodes: int) -> float
     against blended fields: inlet run at 128^3, 100 RK4 steps, 10,000 particles
     0.62 and 4.4 ms, 200,000 2.5 and 7.0, 1M 7.9 and 8.9, 2M 15.8 and 12.3;
     periodic run at 32^3, 30,000 particles 0.65 and 0.97 ms, 100,000 1.5 and 1.1."""
-    evals = {L.JT_EULER: 1, L.JT_RK2: 2}.get(integrator, 4)
-    return 10.0 * evals * n * n_steps / (7.8 * (int(uid[-1]) + 1) * nodes + 3.5e8)
+    return 10.0 * L.EVALS[integrator] * n * n_steps / (7.8 * (int(uid[-1]) + 1) * nodes + 3.5e8)
 
 
 def _stage_numbers(entries) -> np.ndarray:
