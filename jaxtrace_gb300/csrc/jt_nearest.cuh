@@ -121,7 +121,9 @@ __host__ inline NearestLists nearest_lists(const jt_nearest_field& F) {
     float widest = 0.0f;  // the rim of a flat axis is that of the widest live one
     for (int a = 0; a < 3; ++a)
         if (F.cells[a] > 1 && F.inv_cell[a] > 0.0f) widest = fmaxf(widest, 0.5f / F.inv_cell[a]);
-    if (!(widest > 0.0f) || !isfinite(widest)) return g;
+    // the margin of the lists, 1e-5 of a squared distance of that size, has to lie
+    // far above the rounding of squares next to float32's smallest (2^-150)
+    if (!(widest >= 1e-15f) || !isfinite(widest)) return g;
     int64_t cells = 1;
     for (int a = 0; a < 3; ++a) {
         if (F.inv_cell[a] > 0.0f) {
