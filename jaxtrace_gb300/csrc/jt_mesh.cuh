@@ -222,7 +222,8 @@ __device__ __forceinline__ float filter_bary(const V3& q, const uint32_t (&w)[8]
     const float b2 = fmaf(px, b.y, fmaf(py, c.x, pz * c.y));
     const float b3 = fmaf(px, d.x, fmaf(py, d.y, pz * e.x));
     slack = e.y;
-    // minima that let a NaN query through: the full test decides
+    // NaN for a NaN query, which `>= -slack` rejects, as the full test would; a single
+    // NaN, from a query at infinity, is passed over: the full test decides
     return fminf(fminf(1.0f - (b1 + b2 + b3), b1), fminf(b2, b3));
 }
 
@@ -434,15 +435,6 @@ struct MeshFieldT {
             node = (int)(w >> 8) + __popc(m & ((1u << oct) - 1u));
         }
         return __ldg(reinterpret_cast<const int2*>(F.dtab) + node);
-    }
-
-    __device__ __forceinline__ bool slot_test(const V3& q, int slot, float4& b, int4& cn) const {
-        const char* rec = loc + slots + (int64_t)slot * 64;
-        uint32_t g0[8], g1[8];
-        ldg256(rec, g0);
-        ldg256(rec + 32, g1);
-        cn = make_int4((int)g1[4], (int)g1[5], (int)g1[6], (int)g1[7]);
-        return slot_bary<EXACT>(q, g0, g1, b);
     }
 
     // First candidate of the list oc that holds the query (…optimized.py:309-360).
