@@ -395,7 +395,8 @@ class _DeviceField:
         e = self.blend_at(t)
         blend = L.Blend.from_buffer_copy(e.tobytes())
         status = torch.zeros(1, dtype=torch.int32, device="cuda")
-        L.check(L.load().jt_field_sample(C.byref(self._field_for(q.shape[0], 1)), C.byref(blend),
+        field = self._cfield if self._records else self._field_for(q.shape[0], 1)
+        L.check(L.load().jt_field_sample(C.byref(field), C.byref(blend),
                                          self._default_arith() if arith is None else int(arith),
                                          L.ptr(q), L.ptr(out), q.shape[0], L.ptr(status), L.stream_ptr()))
         return out if is_tensor else out.cpu().numpy()
