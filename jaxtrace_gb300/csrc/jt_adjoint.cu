@@ -208,7 +208,8 @@ struct StepRec {
 // to blending the pair records) and the vector-Jacobian products.
 //
 // The L1 bounds it (85 % with node records, 72 loads of a warp a step; issue
-// 35 %), so quads, which blend three times the bytes, pay: 40 loads, and 15.0 ->
+// 35 %), so quads, which blend three times the bytes, pay where a
+// node has a particle (the caller's choice): 40 loads, and 15.0 ->
 // 13.2 ms a pass (1M particles x 50 steps at 64^3, both gradients).  What is left
 // (78 %) is the scatter: a lane's 16-byte atomic is a wavefront of its own.  3
 // blocks/SM measured best (2: 13.7, 4: 14.0 ms).

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kBlock) k_sph(jt_sph_params P) {
                         if (cut) {
                             // no support test, and one sum a lane, joined at the
                             // row's end: 4M positions piled at two walls, h = 0.02,
-                            // 18.0 -> 16.3 ms a pass; 21.6 of 32 lanes active (rows of
+                            // 18.0 -> 16.6 ms a pass; 21.6 of 32 lanes active (rows of
                             // different lengths).  Loops unrolled 1 or 4 times and 6
                             // or 8 blocks/SM: no faster
                             float2 sum = make_float2(0.0f, 0.0f);
