@@ -95,13 +95,22 @@ __global__ void __launch_bounds__(kBlock) k_step(Field f, StageBlends sb, StepCo
     report_flags(status, flags);
 }
 
-// Threads per block of a tracking launch whose caller leaves it open: blocks
-// small enough that a few particles reach all 152 SMs, since one thread's chain
-// of evaluations is what such a run waits for.
+// Threads per block of a tracking launch whose caller leaves it open.  One
+// thread's chain of evaluations is what a launch of few particles waits for, so
+// its blocks are those that leave the busiest of the 152 SMs the fewest threads,
+// the larger ones where that is equal; the smallest only while all threads fit
+// the SMs at once, above which they cost locality.  20 RK4 steps on float32
+// pairs at 64^3, blocks of 64, 128 and 256: 2000 particles 79, 81 and 99 us,
+// 50,000 139, 140 and 186, 80,000 216, 235 and 271, 100,000 256, 273 and 273,
+// 150,000 390, 390 and 351, 200,000 485, 483 and 522, 300,000 450, 442 and 436.
 inline int track_block(int64_t n) {
     constexpr int64_t kSms = 152;
     if (n >= 8 * kSms * kBlock) return kBlock;
-    return n >= 4 * kSms * (kBlock / 2) ? kBlock / 2 : kBlock / 4;
+    const auto busiest = [n](int64_t b) { return (n + kSms * b - 1) / (kSms * b) * b; };
+    int b = kBlock;
+    if (busiest(kBlock / 2) < busiest(b)) b = kBlock / 2;
+    if (n < 3 * kSms * kBlock && busiest(kBlock / 4) < busiest(b)) b = kBlock / 4;
+    return b;
 }
 
 inline unsigned grid_blocks(int64_t n) { return (unsigned)((n + kBlock - 1) / kBlock); }
