@@ -1013,12 +1013,14 @@ def _stage_entries(sched, n_steps: int, integrator: int):
 
 def _stage_gain(n: int, n_steps: int, integrator: int, uid, nodes: int) -> float:
     """What gathering blended fields saves a float32 run over what blending them
-    costs: 10 ps an evaluation against 7.8 ps a node and field (a float32 quad,
-    48 B written) and 0.35 ms for the ring and its launches.  Measured, pairs
-    against blended fields: inlet run at 128^3, 100 RK4 steps, 10,000 particles
-    0.62 and 4.4 ms, 200,000 2.5 and 7.0, 1M 7.9 and 8.9, 2M 15.8 and 12.3;
-    periodic run at 32^3, 30,000 particles 0.65 and 0.97 ms, 100,000 1.5 and 1.1."""
-    return 10.0 * L.EVALS[integrator] * n * n_steps / (7.8 * (int(uid[-1]) + 1) * nodes + 3.5e8)
+    costs: 10 ps an evaluation against 9 ps a node and field (a float32 quad,
+    48 B written) and 0.32 ms for the ring and its launches.  Measured, pairs
+    against blended fields, RK4: inlet run at 128^3, 100 steps, 10,000 particles
+    0.62 and 4.4 ms, 200,000 2.5 and 7.0, 1M 7.9 and 8.9, 2M 15.8 and 12.3; walls
+    at 32^3, 100 steps, 30,000 particles 0.63 and 0.89, 100,000 1.37 and 1.13, 20
+    steps, 100,000 0.47 and 0.56, 400,000 0.80 and 0.77; 17^3, 20 steps, 400,000
+    0.70 and 0.75, 1M 1.22 and 0.99."""
+    return 10.0 * L.EVALS[integrator] * n * n_steps / (9.0 * (int(uid[-1]) + 1) * nodes + 3.2e8)
 
 
 def _stage_numbers(entries) -> np.ndarray:
