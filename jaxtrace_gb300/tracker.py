@@ -353,7 +353,7 @@ class ParticleTracker:
         p.block_size = int(self.options.block_size)
         return p
 
-    def _sort_every(self, n: int) -> int:
+    def _sort_every(self, n: int, n_steps: int) -> int:
         """Locality re-sort interval: 100 steps on a regular grid from 2^18
         particles up (16.8M-particle precision workload, 1000 steps: bfloat16 299
         ms at 50, 290 at 100, 289 at 150, 290 at 200, 297 at 300; float32 412, 407,
@@ -361,12 +361,16 @@ class ParticleTracker:
         scattered nodes, whose lookups lose locality sooner, from 2^17 up (64
         steps, octree, 1M particles: 12.9 ms at 8, 12.5 at 16, 12.3 at 32, 12.4 at
         64, 18.1 unsorted; 200,000 particles 4.2 ms at 32 and 4.7 unsorted, 60,000
-        2.35 and 2.30; scattered nodes, 200,000 particles 1.68 and 2.09 ms)."""
+        2.35 and 2.30; scattered nodes, 200,000 particles 1.68 and 2.09 ms).
+        Below 2^18 a short run does not earn its sort back (0.05 to 0.08 ms): sorted
+        and unsorted, 1,572,864 tetrahedra, 132,000 particles 8 steps octree 0.54 and
+        0.48, hash grid 0.68 and 0.63, nodes 0.44 and 0.35; 200,000 particles 16 steps
+        1.18 and 1.25, 1.53 and 1.75, 0.80 and 0.78."""
         se = self.options.sort_every
         if se is None:
             from .fields import OctreeFEMTimeSeriesFieldOptimized, TimeSeriesField
             scattered = isinstance(self._field, (OctreeFEMTimeSeriesFieldOptimized, TimeSeriesField))
-            if n < (1 << (17 if scattered else 18)):
+            if n < (1 << 18) and not (scattered and n >= 1 << 17 and n * n_steps >= 3_000_000):
                 return 0
             if scattered:
                 return 32
@@ -388,7 +392,8 @@ class ParticleTracker:
         comp_zero = comp is None
         if comp is None and self._arith() == L.JT_ARITH_COMPENSATED:
             comp = torch.zeros_like(pos)
-        return _Engine(self, pos, len(times) - 1, dt, sched_dev, status, comp, self._sort_every(pos.shape[0]),
+        return _Engine(self, pos, len(times) - 1, dt, sched_dev, status, comp,
+                       self._sort_every(pos.shape[0], len(times) - 1),
                        ens=ens, sched=sched, comp_zero=comp_zero)
 
     def _run(self, pos, times, dt, k, compact, n_rows, positions, velocities, rows_out=None) -> int:
