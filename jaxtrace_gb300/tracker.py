@@ -50,8 +50,8 @@ class TrackerOptions:
     time_chunk         steps per kernel launch (None: as many as fit)
     sort_every         re-sort particles by cell every k steps for gather
                        locality (None: on regular grids 100 from 2^18 particles
-                       up, on meshes and scattered nodes 32 from 2^17 up; 0:
-                       never)
+                       up, on meshes and scattered nodes 32 from there, and
+                       from 2^17 in longer runs; 0: never)
     sort_bits          cells per axis of that sort, as a power of two
                        (None: 2^7)
     block_size         threads per block of the tracking kernel (0: by the
