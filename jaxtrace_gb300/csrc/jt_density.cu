@@ -439,23 +439,24 @@ constexpr int kKbT = 8;  // the 3-D KDE's grid tile edge
 // Sums run in float32 over at most kKdSpan particles of a thread, all further
 // ones in float64, by way of shared memory (32 float64 sums of a thread's own
 // would take 64 registers).  3,000,017 particles, 100^3 points: 21.4 ms with eight
-// points a thread (64 threads, bound by shared memory), 13.0 ms with 32 and the
-// cells below; with 240 particles in a sum 5 % less time and larger errors.
+// points a thread (64 threads, bound by shared memory, float32 sums of 240
+// particles too), 12.1 ms with 32 and the cells below; with 128 particles in a
+// sum 8 % more time and 8 % less error.
 //
 // The particles summed are those of the cells that meet the tile grown by one
 // radius along each axis, and, where a radius is 5 bandwidths or more (the
 // default), also those within kKdReach radii of the tile: with the finer cells
 // that the estimator then cuts, of which less lies beyond the radius, that keeps
 // the error below that of cells of half a radius: 3,000,017 particles, 100^3
-// points, median 5.9e-8 against 7.0e-8.  The grown tile alone would take 4 % less
-// time with 8.8e-8, a rim of 1.2 radii 8 % more with 5.2e-8.  The rows of cells
-// are listed first, a row a thread and step, and their particles then dealt out
-// in whole chunks: walking the rows one by one cost as much as the finer cells
-// saved.
+// points, median 6.4e-8 against 7.0e-8; 200,000, 81^3, 5.7e-8 against 9.5e-8.  The
+// grown tile alone would take 4 % less time with 8.8e-8, a rim of 1.2 radii 8 %
+// more with 6.0e-8.  The rows of cells are listed first, a row a thread and step,
+// and their particles then dealt out in whole chunks: walking the rows one by one
+// cost as much as the finer cells saved.
 constexpr int kKdThreads = 128;
 constexpr int kKdGroups = kKdThreads / 16;
 constexpr int kKdChunk = 256;   // particles in shared memory: 3 x 256 x 32 B = 24 KB
-constexpr int kKdSpan = 128;    // particles in a float32 sum, at most
+constexpr int kKdSpan = 240;    // particles in a float32 sum, at most
 constexpr float kKdReach = 1.1f, kKdReachFrom = 4.999f;
 constexpr int kKdRows = 4 * kKdThreads;  // rows of cells listed at a time
 static_assert(kKdGroups * kKbT * kKbT * kKbT <= 3 * kKdChunk * kKbT, "the groups' sums fit the factors' memory");
