@@ -122,11 +122,14 @@ __device__ __forceinline__ float2 sph_shape2(float2 q) {
 // support adds exactly 0.  The cubic spline is the smaller of its two branches
 // at any q: 1 - 1.5 q^2 + 0.75 q^3 less (2 - q)+^3 / 4 is (q - 1)^3 up to q = 2
 // and positive beyond.  Both are halved, which is exact and saves a
-// multiplication, and round as sph_shape does.  (The one formula
-// (2 - q)+^3 / 4 - (1 - q)+^3 cancels below q = 1: rms error of a term 5.1e-8 of
-// the kernel's height there against 3.0e-8, for 3 % of the time: 4M uniform
-// positions, h = 0.02, 8.61 ms against 8.88.)  d2 must not be 0: the sum adds
-// `tiny`, 1e-14 h^2, which moves no q by more than 1e-7.
+// multiplication, and q^2 comes from d2, which saves another and the rounding of
+// the root.  The rms error of a term, in units of the kernel's height: 1.7e-8
+// below q = 0.05, 2.1e-8 to 0.5, 3.6e-8 to 0.95, 2.6e-8 from 1.05 to 1.5; 1.7e-8,
+// 2.3e-8, 4.3e-8 and 2.8e-8 with sph_shape.  (The one formula
+// (2 - q)+^3 / 4 - (1 - q)+^3 cancels below q = 1, 4.3e-8, 4.5e-8 and 4.8e-8 there,
+// and takes the same time: 4M uniform positions, h = 0.02, 8.61 ms against 8.59.)
+// d2 must not be 0: the sum adds `tiny`, 1e-14 h^2, which moves no q by more than
+// 1e-7.
 template <int KERN>
 constexpr float kSphCut = KERN == JT_SPH_CUBIC ? 2.0f : 1.0f;
 
@@ -134,9 +137,9 @@ template <int KERN>
 __device__ __forceinline__ float2 sph_cut2(float2 d2, float inv) {
     const float2 dist = __fmul2_rn(d2, make_float2(rsqrtf(d2.x), rsqrtf(d2.y)));
     if (KERN == JT_SPH_CUBIC) {
-        const float2 q = __fmul2_rn(dist, splat(inv));
-        const float2 inner = __ffma2_rn(__fmul2_rn(q, q), __ffma2_rn(splat(0.375f), q, splat(-0.75f)), splat(0.5f));
-        const float2 u = __ffma2_rn(splat(-0.5f), q, splat(1.0f));
+        const float2 inner = __ffma2_rn(__fmul2_rn(d2, splat(inv * inv)),
+                                        __ffma2_rn(dist, splat(0.375f * inv), splat(-0.75f)), splat(0.5f));
+        const float2 u = __ffma2_rn(dist, splat(-0.5f * inv), splat(1.0f));
         const float2 a = make_float2(fmaxf(u.x, 0.0f), fmaxf(u.y, 0.0f));
         const float2 outer = __fmul2_rn(__fmul2_rn(a, a), a);
         return make_float2(fminf(inner.x, outer.x), fminf(inner.y, outer.y));
@@ -238,7 +241,7 @@ __global__ void __launch_bounds__(kBlock) k_sph(jt_sph_params P) {
                         if (cut) {
                             // no support test, and one sum a lane, joined at the
                             // row's end: 4M positions piled at two walls, h = 0.02,
-                            // 18.0 -> 16.6 ms a pass; 21.6 of 32 lanes active (rows of
+                            // 18.0 -> 15.9 ms a pass; 21.6 of 32 lanes active (rows of
                             // different lengths).  Loops unrolled 1 or 4 times and 6
                             // or 8 blocks/SM: no faster
                             float2 sum = make_float2(0.0f, 0.0f);
@@ -718,7 +721,7 @@ using namespace jt;
 // 47.4 and 49.0 us; 1.1 (1M, Wendland, h = 0.005) 78.3 and 87.0; 3.9 (1M,
 // h = 0.014) 727 and 713; 4.4 (4M, Wendland, h = 0.005) 417 and 427; 6.8 (4M,
 // h = 0.005) 1050 and 1024, (Wendland, h = 0.01) 951 and 941; 21 (4M, h = 0.02)
-// 9616 and 8918; 2-D, 20,000: 4.4 11.3 and 11.5, 7.5 16.6 and 16.5.
+// 9616 and 8594; 2-D, 20,000: 4.4 11.3 and 11.5, 7.5 16.6 and 16.5.
 constexpr double kSphCutRow = 6.0;
 
 static bool sph_cut(const jt_sph_params& p) {

@@ -119,3 +119,12 @@ def test_rows_choose_the_loop(kind, dims):
         assert np.allclose(out[1], out[2], rtol=1e-5)
     assert np.array_equal(got[0.01][1], got[0.01][2])          # one or two candidates a row: the same loop's terms
     assert not np.array_equal(got[1.0][1], got[1.0][2])        # thousands a row: the other
+
+
+@pytest.mark.parametrize("lo,hi", [(0.05, 0.5), (0.5, 0.95), (1.05, 1.5), (1.5, 1.99)])
+def test_terms_round_as_the_spline_of_the_tested_loop(lo, hi):
+    """The rounding of q, at most 8 2^-24 of it, times the slope (at most 1 at
+    q = 2/3), and four roundings of values up to 1."""
+    r, got = _one_term("cubic_spline", lo, hi)
+    want = np.where(r <= 1, 1 - 1.5 * r ** 2 + 0.75 * r ** 3, 0.25 * (2 - r) ** 3)
+    assert np.abs(got - want).max() <= 12 * 2.0 ** -24
